@@ -331,14 +331,22 @@ int build_tables(swg_adjoint ad) {
   return SWG_OK;
 }
 
-// aux arrays of the same set as the model's, of value type T
-template <class T> int alloc_aux_like(swg_adjoint ad, AuxViewT<T> &d) {
+// aux arrays of the same set as the model's, of value type T.  share: the
+// set of another stage of the same tape, whose words of the fixed-point sums
+// serve this one too: a stage's own passes read them, the adjoint does not.
+template <class T>
+int alloc_aux_like(swg_adjoint ad, AuxViewT<T> &d,
+                   const AuxViewT<T> *share = nullptr) {
   swg_model md = ad->model;
   const AuxView &a = md->aux;
   const size_t C = md->mesh->ncells, E = md->mesh->nedges,
                V = md->mesh->nvertices, K = md->mesh->nlayers,
                T_ = md->params.ntracers;
   auto &A = ad->allocs;
+  // F Q itself: without the words, and for dual numbers
+  const double *G = a.G;
+  if (std::is_same<T, Dual>::value && a.FGx)
+    G = reinterpret_cast<const double *>(a.FGx);
   struct {
     const double *on;
     size_t n;
@@ -347,12 +355,26 @@ template <class T> int alloc_aux_like(swg_adjoint ad, AuxViewT<T> &d) {
            {a.z4, V * K, &d.z4},     {a.div, C * K, &d.div},
            {a.ke, C * K, &d.ke},     {a.d4, C * K, &d.d4},
            {a.ntr, T_ * C * K, &d.ntr}, {a.lap, T_ * C * K, &d.lap},
-           {a.F, E * K, &d.F},       {a.G, E * K, &d.G},
+           {a.F, E * K, &d.F},       {G, E * K, &d.G},
            {a.Q, E * K, &d.Q},       {a.mh, E * K, &d.mh},
            {a.u2, E * K, &d.u2},     {a.d2u, E * K, &d.d2u}};
   for (auto &x : t)
     if (x.on)
       TRY(zal(A, x.n, x.p));
+  if constexpr (std::is_same<T, double>::value) {
+    if (share) {
+      d.FGx = share->FGx;
+      d.nx = share->nx;
+      d.lx = share->lx;
+    } else {
+      if (a.FGx)
+        TRY(zal(A, 2 * E * K, reinterpret_cast<double **>(&d.FGx)));
+      if (a.nx)
+        TRY(zal(A, T_ * C * K, reinterpret_cast<double **>(&d.nx)));
+      if (a.lx)
+        TRY(zal(A, T_ * C * K, reinterpret_cast<double **>(&d.lx)));
+    }
+  }
   d.d2u4 = d.d2u;
   if (a.d2u4 && a.d2u4 != a.d2u) // 1/max(dv, dc/4) differs from 1/dv
     TRY(zal(A, E * K, &d.d2u4));
@@ -368,12 +390,12 @@ int alloc_tape(swg_adjoint ad, int b, int s) {
                V = md->mesh->nvertices, K = md->mesh->nlayers;
   AuxView &t = ad->tp[b].taux[s];
   auto &A = ad->allocs;
-  TRY(alloc_aux_like(ad, t));
+  const AuxView &t0 = ad->tp[b].taux[0];
+  TRY(alloc_aux_like(ad, t, s > 0 ? &t0 : nullptr));
   if (md->view.do_vn) {
     TRY(zal(A, V * K, &t.rhv));
-    // the last stage's PV sum is written only when the step's final
-    // passes run (a taped advance); the adjoint of a tape from a state
-    // recomputes it (adjoint_step's last_s1)
+    // the last stage's PV sum comes from the step's final passes (a taped
+    // advance) or, where they do not run, from a pass of its own
     TRY(zal(A, E * K, &t.S1));
   }
   if (md->params.ntracers > 0)
@@ -468,6 +490,12 @@ void adj_tendency(swg_adjoint ad, const double *h, const double *vn,
                   cudaStream_t st) {
   swg_model md = ad->model;
   launch_aux(md->mesh->view, md->view, md->aux, h, vn, tr, st, &md->fork);
+  // the PV sums go to the edge pass's own work array: each thread reads its
+  // S1 before it writes that element of lQ
+  AuxView aux = md->aux;
+  aux.S1 = ad->aw.lQ;
+  if (md->view.do_vn && !md->view.off_pv)
+    launch_pv_sum(md->mesh->view, aux, st);
   AdjIO io{};
   io.h = h;
   io.vn = vn;
@@ -478,7 +506,7 @@ void adj_tendency(swg_adjoint ad, const double *h, const double *vn,
   io.lh = out->h;
   io.lvn = out->vn;
   io.ltr = out->tr;
-  adj_passes(ad, md->aux, io, st);
+  adj_passes(ad, aux, io, st);
 }
 
 void lincomb(swg_state y, swg_state x1, swg_state x2, double a, double b,
@@ -507,6 +535,8 @@ int tape_step(swg_adjoint ad, TapeSlot &tp, double dt, swg_state out,
       const double *h, *vn, *tr;
       stage_ptrs(ad, tp, s, &h, &vn, &tr);
       launch_aux(md->mesh->view, pv, tp.taux[s], h, vn, tr, st, &md->fork);
+      if (pv.do_vn && !pv.off_pv)
+        launch_pv_sum(md->mesh->view, tp.taux[s], st);
       continue;
     }
     TRY(tape_stage_copy(ad, tp, s, out, st));
@@ -531,19 +561,14 @@ int tape_step(swg_adjoint ad, TapeSlot &tp, double dt, swg_state out,
 // lamX_s = lamX_{s+1} + J(X_s)^T mu_s and
 // mu_{s-1} = dt b_{s-1} lamX_s + a_s mu_s; the step's adjoint is lamX_0.
 // The output passes accumulate lamX in lacc and form mu_{s-1} from it.
-// last_s1: the tape was written by a taped advance, whose last stage ran
-// its final passes and taped that stage's PV sum too
-int adjoint_step(swg_adjoint ad, const TapeSlot &tp, double dt, bool last_s1,
+int adjoint_step(swg_adjoint ad, const TapeSlot &tp, double dt,
                  cudaStream_t st) {
   const int ns = ad->ns;
   if (ns % 2 != 0)
     lincomb(ad->mu, ad->lam, nullptr, dt * step_rkb(ad)[ns - 1], 0.0,
             (long long)words(ad->model), st);
   for (int s = ns - 1; s >= 0; --s) {
-    AuxView aux = tp.taux[s];
-    if (s == ns - 1 && !last_s1)
-      aux.S1 = nullptr;
-    adj_passes(ad, aux, stage_io(ad, tp, s, dt), st);
+    adj_passes(ad, tp.taux[s], stage_io(ad, tp, s, dt), st);
   }
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? SWG_OK : cuda_fail(err, "swg_adjoint: adjoint step");
@@ -829,12 +854,12 @@ int run_action(swg_adjoint ad, const AdjAction &a, cudaStream_t st, bool two) {
     // forcing), replayed from a graph captured on first use
     rc = replay(ad, tp.tape_adj, st, [&](cudaStream_t cs) {
       TRY(tape_step(ad, tp, ad->dt, nullptr, cs));
-      return adjoint_step(ad, tp, ad->dt, false, cs);
+      return adjoint_step(ad, tp, ad->dt, cs);
     });
   } else {
     // a reversal without its own tape follows a taped advance into tp
     rc = replay(ad, tp.adj, st, [&](cudaStream_t cs) {
-      return adjoint_step(ad, tp, ad->dt, true, cs);
+      return adjoint_step(ad, tp, ad->dt, cs);
     });
   }
   if (rc == SWG_OK && two && (e = cudaEventRecord(tp.free_ev, st)) != cudaSuccess)
@@ -1462,6 +1487,10 @@ extern "C" int swg_adj_memory(swg_adjoint ad, long long *snapshot_bytes,
   size_t tape = 0;
   for (int s = 0; s < ad->ns; ++s)
     tape += aux_bytes(ad->tp[0].taux[s], C, E, V, K, T);
+  const AuxView &t0 = ad->tp[0].taux[0];
+  // words of the fixed-point sums, one set for all stages
+  tape += ((t0.FGx ? 2 * E : 0) + ((t0.nx != nullptr) + (t0.lx != nullptr)) *
+           T * C) * K * sizeof(fx_t);
   tape += size_t(ad->ns + 1) * state; // stage inputs and accumulator
   if (snapshot_bytes)
     *snapshot_bytes = (long long)state;

@@ -78,6 +78,101 @@ int dalloc(std::vector<void *> &allocs, size_t n, double **dev) {
   return SWG_OK;
 }
 
+int check_launch(const char *what) {
+  cudaError_t err = cudaGetLastError();
+  return err == cudaSuccess ? SWG_OK : cuda_fail(err, what);
+}
+
+// The tables of fixed-point terms, converted on the device from the uploaded
+// index and weight tables.
+__global__ void k_edge_terms(MeshView m, int ne, FxSlot *out, long long *start,
+                             unsigned *bad) {
+  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (e >= m.nedges)
+    return;
+  long long sum = 0;
+  unsigned flag = 0;
+  for (int j = 0; j < ne; ++j) {
+    const FxSlot t{m.eoe[ne * e + j], fx_weight(m.woe[ne * e + j], flag)};
+    out[ne * e + j] = t;
+    sum += t.w.hi;
+  }
+  start[e] = fx_start(sum);
+  if (flag)
+    atomicOr(bad, flag);
+}
+__global__ void k_cell_terms(MeshView m, const double *r4, FxSlot *out) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i < 6LL * m.ncells)
+    out[i] = FxSlot{m.nbc[i], fx_table_weight(r4[i])};
+}
+// mv.fxe, mv.fxe0: left null when a weight is out of range
+int edge_terms_table(std::vector<void *> &allocs, MeshView &mv, int ne) {
+  double *t = nullptr, *s = nullptr, *b = nullptr;
+  TRY(dalloc(allocs, size_t(ne) * mv.nedges * (sizeof(FxSlot) / 8), &t));
+  TRY(dalloc(allocs, mv.nedges, &s));
+  TRY(dalloc(allocs, 1, &b));
+  FxSlot *slots = reinterpret_cast<FxSlot *>(t);
+  long long *start = reinterpret_cast<long long *>(s);
+  unsigned *bad = reinterpret_cast<unsigned *>(b), bad_h = 0;
+  k_edge_terms<<<unsigned((mv.nedges + 255) / 256), 256>>>(mv, ne, slots,
+                                                           start, bad);
+  TRY(check_launch("edge terms table"));
+  cudaError_t err = cudaMemcpy(&bad_h, bad, 4, cudaMemcpyDeviceToHost);
+  if (err != cudaSuccess)
+    return cuda_fail(err, "edge terms table");
+  if (!bad_h) {
+    mv.fxe = slots;
+    mv.fxe0 = start;
+  }
+  return SWG_OK;
+}
+int cell_terms_table(std::vector<void *> &allocs, const MeshView &m,
+                     ModelView &pv) {
+  double *t = nullptr;
+  const long long n = 6LL * m.ncells;
+  TRY(dalloc(allocs, size_t(n) * (sizeof(FxSlot) / 8), &t));
+  FxSlot *slots = reinterpret_cast<FxSlot *>(t);
+  k_cell_terms<<<unsigned((n + 255) / 256), 256>>>(m, pv.r4, slots);
+  TRY(check_launch("cell terms table"));
+  // finished before a caller's stream reads it
+  cudaError_t err = cudaStreamSynchronize(nullptr);
+  if (err != cudaSuccess)
+    return cuda_fail(err, "cell terms table");
+  pv.r4x = slots;
+  return SWG_OK;
+}
+
+// The words of the fixed-point sums: ne pairs for the fluxes, nt each for the
+// tracers and (lap) their Laplacians.  They only speed the sums up, so they
+// are left out (all null, FP64 sums) where they would take more than a
+// quarter of the free device memory: a model that fitted without them must
+// leave room for the states and steppers that come after it.  `must`: as
+// given, without that rule.
+int alloc_words(std::vector<void *> &allocs, size_t ne, size_t nt, bool lap,
+                bool must, AuxView &a) {
+  const size_t nl = lap ? nt : 0;
+  if (!must) {
+    size_t free_b = 0, total_b = 0;
+    cudaError_t err = cudaMemGetInfo(&free_b, &total_b);
+    if (err != cudaSuccess)
+      return cuda_fail(err, "cudaMemGetInfo (work arrays)");
+    if ((2 * ne + nt + nl) * sizeof(fx_t) > free_b / 4)
+      return SWG_OK;
+  }
+  double *f = nullptr, *n = nullptr, *l = nullptr;
+  if (ne)
+    TRY(dalloc(allocs, 2 * ne, &f));
+  if (nt)
+    TRY(dalloc(allocs, nt, &n));
+  if (nl)
+    TRY(dalloc(allocs, nl, &l));
+  a.FGx = reinterpret_cast<fx_t *>(f);
+  a.nx = reinterpret_cast<fx_t *>(n);
+  a.lx = reinterpret_cast<fx_t *>(l);
+  return SWG_OK;
+}
+
 void free_all(std::vector<void *> &allocs) {
   for (void *p : allocs)
     cudaFree(p);
@@ -101,10 +196,6 @@ bool all_equal(const int *a, size_t n, int x) {
 
 cudaStream_t as_stream(void *s) { return static_cast<cudaStream_t>(s); }
 
-int check_launch(const char *what) {
-  cudaError_t err = cudaGetLastError();
-  return err == cudaSuccess ? SWG_OK : cuda_fail(err, what);
-}
 
 } // namespace
 } // namespace swg
@@ -303,6 +394,7 @@ extern "C" int swg_mesh_create(const swg_mesh_desc *d, swg_mesh *out) try {
       (rc = upload(A, inv_dv4.data(), E, &mv.inv_dv4)) ||
       (rc = upload(A, eoe.data(), size_t(NE) * E, &mv.eoe)) ||
       (rc = upload(A, woe.data(), size_t(NE) * E, &mv.woe)) ||
+      (rc = edge_terms_table(A, mv, NE)) ||
       (rc = upload(A, m->scale2_h.data(), E, &mv.scale2)) ||
       (rc = upload(A, m->scale4_h.data(), E, &mv.scale4)) ||
       (rc = upload(A, d->area_cell, C, &mv.area_cell_d)) ||
@@ -535,6 +627,7 @@ extern "C" int swg_model_create_ex(swg_mesh mesh, const swg_params *p,
       (rc = upload(A, kd2.data(), 6 * C, &pv.kd2)) ||
       (rc = upload(A, r4.data(), 6 * C, &pv.r4)) ||
       (rc = upload(A, r4s.data(), C, &pv.r4sum)) ||
+      (T > 0 && pv.tr_del4 && (rc = cell_terms_table(A, mesh->view, pv))) ||
       (!r4f.empty() && (rc = upload(A, r4f.data(), C, &pv.r4f)))) {
     swg_model_destroy(md);
     return rc;
@@ -543,6 +636,12 @@ extern "C" int swg_model_create_ex(swg_mesh mesh, const swg_params *p,
   const bool vn = pv.do_vn;
   const bool vdiss = vn && (pv.vel_del2 || pv.vel_del4);
   const bool v4 = vn && pv.vel_del4;
+  const FxUse fx = fx_use(mesh, pv);
+  if ((rc = alloc_words(A, fx.pv ? E * K : 0, fx.tr ? T * C * K : 0,
+                        pv.tr_del4, mesh->fx_given, a)) != SWG_OK) {
+    swg_model_destroy(md);
+    return rc;
+  }
   struct Need {
     bool on;
     size_t n;
@@ -554,7 +653,7 @@ extern "C" int swg_model_create_ex(swg_mesh mesh, const swg_params *p,
       {vn, E * K, &a.u2},
       {T > 0, T * C * K, &a.ntr},
       {T > 0 && pv.tr_del4, T * C * K, &a.lap},
-      {true, E * K, &a.F},      {vn, E * K, &a.G},
+      {true, E * K, &a.F},      {vn && !a.FGx, E * K, &a.G},
       // the mean thickness is kept always: the per-field tendency calls
       // read the last auxiliary state's (the reference's m_mean_h_edge)
       {vn, E * K, &a.Q},        {true, E * K, &a.mh},

@@ -87,8 +87,10 @@ __device__ __forceinline__ void run_pass(int pass, const Member &M, int stage,
 
 // Passes [pass0, pass1] of stage `stage` for all members.  prefix[pass] has
 // nmem+1 entries: virtual-block offsets of the members in that pass.
-template <int NE, int ITEMS>
-__global__ void __launch_bounds__(512)
+// BLOCK: threads per block; 24 resident warps per SM (80 registers) where the
+// block allows them.
+template <int NE, int ITEMS, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, BLOCK > 256 ? 1 : 768 / BLOCK)
     k_batch(const Member *__restrict__ mem, int nmem,
             const unsigned *__restrict__ prefix, int stage, int pass0,
             int pass1, BatchSync *bs, long long limit) {
@@ -120,6 +122,20 @@ __global__ void __launch_bounds__(512)
   }
 }
 
+// The member a virtual block belongs to: the last m with pre[m] <= vb.
+__device__ __forceinline__ int member_of(const unsigned *pre, int nmem,
+                                         unsigned vb) {
+  int lo = 0, hi = nmem;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (pre[mid] <= vb)
+      lo = mid;
+    else
+      hi = mid;
+  }
+  return lo;
+}
+
 // One pass of one stage for all members (the per-pass launch shape), with
 // the pass fixed at compile time: each pass kernel is compiled on its own,
 // so a light pass does not carry the registers of the heaviest one and
@@ -132,27 +148,66 @@ __global__ void __launch_bounds__(512)
   const unsigned *pre = prefix + PASS * (nmem + 1);
   const unsigned nvb = pre[nmem];
   for (unsigned vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-    int lo = 0, hi = nmem;
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (pre[mid] <= vb)
-        lo = mid;
-      else
-        hi = mid;
-    }
+    const int lo = member_of(pre, nmem, vb);
     const Member &M = mem[lo];
     const unsigned n = M.units[PASS];
     const unsigned first = (vb - pre[lo]) * vbsize + threadIdx.x;
 #pragma unroll
     for (int it = 0; it < ITEMS; ++it) {
       const unsigned i = first + it * blockDim.x;
-      if (i < n)
+      if (i >= n)
+        continue;
+      // no member keeps the words of the heavy passes' fixed-point sums
+      if (PASS == P_AUX2)
+        pt_aux2<double, -2>(M.m, M.p, M.a, M.aux2_base + i);
+      else if (PASS == P_EDGE_FINAL)
+        pt_edge_final<NE, double, 0>(M.m, M.p, M.a, M.stage[stage], i);
+      else if (PASS == P_CELL_FINAL)
+        pt_cell_final<double, 0>(M.m, M.p, M.a, M.stage[stage], i);
+      else
         run_pass<NE>(PASS, M, stage, i);
     }
   }
 }
 
-template <int NE, int ITEMS> void *pass_kernel(int pass) {
+// The passes with fixed-point sums (P_AUX2, P_EDGE_FINAL, P_CELL_FINAL, and
+// P_PV_SUM) of batches whose members (or some of them) keep the words, in
+// the single-instance kernels' shape whatever the configuration's block:
+// 2^shift blocks of HTPB threads per virtual block, HEAVY_ITEMS elements a
+// thread (finding the member and reading its descriptor is a chain of loads
+// at each block's start).
+constexpr int HEAVY_ITEMS = 2;
+template <int PASS> constexpr int heavy_blocks() {
+  return PASS == P_AUX2 ? HEAVY_AUX2_BLOCKS
+         : PASS == P_CELL_FINAL ? HEAVY_CELL_BLOCKS
+                                : HEAVY_EDGE_BLOCKS;
+}
+template <int NE, int PASS>
+__global__ void __launch_bounds__(HTPB, heavy_blocks<PASS>())
+    k_batch_heavy(const Member *__restrict__ mem, int nmem,
+                  const unsigned *__restrict__ prefix, int stage, int shift) {
+  __shared__ fx_t sm[PASS == P_CELL_FINAL ? 2 * TR_SLOTS * HTPB : 1];
+  constexpr int DOMAIN = PASS == P_PV_SUM ? P_EDGE_FINAL : PASS;
+  const unsigned *pre = prefix + DOMAIN * (nmem + 1);
+  const unsigned vb = blockIdx.x >> shift;
+  const int lo = member_of(pre, nmem, vb);
+  const Member &M = mem[lo];
+  const unsigned n = M.units[DOMAIN];
+  unsigned i = (blockIdx.x - (pre[lo] << shift)) * (HTPB * HEAVY_ITEMS) +
+               threadIdx.x;
+#pragma unroll 1
+  for (int it = 0; it < HEAVY_ITEMS && i < n; ++it, i += HTPB) {
+    if (PASS == P_CELL_FINAL)
+      pt_cell_final<double, -1, true>(M.m, M.p, M.a, M.stage[stage], i,
+                                      sm + threadIdx.x, HTPB);
+    else if (PASS == P_PV_SUM)
+      pt_pv_sum<NE>(M.m, M.a, i);
+    else
+      run_pass<NE>(PASS, M, stage, i);
+  }
+}
+
+template <int NE, int ITEMS> void *light_kernel(int pass) {
   switch (pass) {
   case P_VERTEX:
     return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_VERTEX>);
@@ -168,24 +223,61 @@ template <int NE, int ITEMS> void *pass_kernel(int pass) {
     return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_CELL_FINAL>);
   }
 }
+template <int NE> void *heavy_kernel(int pass) {
+  switch (pass) {
+  case P_AUX2:
+    return reinterpret_cast<void *>(&k_batch_heavy<NE, P_AUX2>);
+  case P_EDGE_FINAL:
+    return reinterpret_cast<void *>(&k_batch_heavy<NE, P_EDGE_FINAL>);
+  case P_PV_SUM:
+    return reinterpret_cast<void *>(&k_batch_heavy<NE, P_PV_SUM>);
+  default:
+    return reinterpret_cast<void *>(&k_batch_heavy<NE, P_CELL_FINAL>);
+  }
+}
+
+unsigned batch_heavy_passes(const swg_model_s *md) {
+  const AuxView &a = md->aux;
+  return (a.lx ? 1u << P_AUX2 : 0u) | (a.FGx ? 1u << P_EDGE_FINAL : 0u) |
+         (a.nx ? 1u << P_CELL_FINAL : 0u) | 1u << P_PV_SUM;
+}
+
+// One pass over nvb virtual blocks of block x items elements (block a power
+// of two from 128).
+static int launch_pass(const Member *mem, int nmem, const unsigned *prefix,
+                       int ne, int pass, unsigned heavy, int stage,
+                       unsigned nvb, int block, int items, cudaStream_t st) {
+  if (nvb == 0)
+    return SWG_OK;
+  void *fn;
+  int shift = 0;
+  if (heavy >> pass & 1) {
+    fn = ne == 8 ? heavy_kernel<8>(pass) : heavy_kernel<10>(pass);
+    while ((HTPB * HEAVY_ITEMS << shift) < block * items)
+      ++shift;
+    nvb <<= shift;
+    block = HTPB;
+  } else if (items == 2) {
+    fn = ne == 8 ? light_kernel<8, 2>(pass) : light_kernel<10, 2>(pass);
+  } else {
+    fn = ne == 8 ? light_kernel<8, 1>(pass) : light_kernel<10, 1>(pass);
+  }
+  void *args[] = {&mem, &nmem, &prefix, &stage, &shift};
+  cudaError_t err = cudaLaunchKernel(fn, dim3(nvb), dim3(block), args, 0, st);
+  if (err != cudaSuccess)
+    return cuda_fail(err, "batched passes: launch");
+  ++g_launches;
+  return SWG_OK;
+}
 
 int batch_launch_passes(const Member *mem, int nmem, const unsigned *prefix,
                         const unsigned *prefix_h, int ne, int items,
-                        int pass0, int pass1, int stage, cudaStream_t st) {
+                        unsigned heavy, int pass0, int pass1, int stage,
+                        cudaStream_t st) {
   for (int pass = pass0; pass <= pass1; ++pass) {
-    const unsigned nvb = prefix_h[pass * (nmem + 1) + nmem];
-    if (nvb == 0)
-      continue;
-    void *args[] = {&mem, &nmem, &prefix, &stage};
-    void *fn = items == 2 ? (ne == 8 ? pass_kernel<8, 2>(pass)
-                                     : pass_kernel<10, 2>(pass))
-                          : (ne == 8 ? pass_kernel<8, 1>(pass)
-                                     : pass_kernel<10, 1>(pass));
-    cudaError_t err =
-        cudaLaunchKernel(fn, dim3(nvb), dim3(256), args, 0, st);
-    if (err != cudaSuccess)
-      return cuda_fail(err, "batched passes: launch");
-    ++g_launches;
+    const int domain = pass == P_PV_SUM ? P_EDGE_FINAL : pass;
+    TRY(launch_pass(mem, nmem, prefix, ne, pass, heavy, stage,
+                    prefix_h[domain * (nmem + 1) + nmem], 256, items, st));
   }
   return SWG_OK;
 }
@@ -216,6 +308,7 @@ static const int kNumConfigs = sizeof(kConfigs) / sizeof(kConfigs[0]);
 
 struct swg_batch_s {
   int nmem, kind, nstages, ne;
+  unsigned heavy = 0; // passes with fixed-point sums in some member
   std::vector<swg_model> models;
   std::vector<swg_state> states, tend, acc, p0, p1;
   std::vector<double> rka, rkb, rkc;
@@ -327,32 +420,17 @@ int upload_members(swg_batch b, double dt) {
   return SWG_OK;
 }
 
-template <int NE, int ITEMS> void *kernel_ptr() {
-  return reinterpret_cast<void *>(&k_batch<NE, ITEMS>);
-}
-
-void *pick_kernel(int ne, int items) {
-  if (ne == 8)
-    return items == 1 ? kernel_ptr<8, 1>() : kernel_ptr<8, 2>();
-  return items == 1 ? kernel_ptr<10, 1>() : kernel_ptr<10, 2>();
-}
-
-template <int NE, int ITEMS> void *pass_kernel_ptr(int pass) {
-  switch (pass) {
-  case P_VERTEX: return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_VERTEX>);
-  case P_CELL1: return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_CELL1>);
-  case P_EDGE1: return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_EDGE1>);
-  case P_AUX2: return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_AUX2>);
-  case P_EDGE_FINAL:
-    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_EDGE_FINAL>);
-  default: return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_CELL_FINAL>);
+template <int NE, int ITEMS> void *kernel_ptr(int block) {
+  switch (block) {
+  case 128: return reinterpret_cast<void *>(&k_batch<NE, ITEMS, 128>);
+  case 256: return reinterpret_cast<void *>(&k_batch<NE, ITEMS, 256>);
+  default: return reinterpret_cast<void *>(&k_batch<NE, ITEMS, 512>);
   }
 }
-
-void *pick_pass_kernel(int ne, int items, int pass) {
+void *pick_kernel(int ne, int items, int block) {
   if (ne == 8)
-    return items == 1 ? pass_kernel_ptr<8, 1>(pass) : pass_kernel_ptr<8, 2>(pass);
-  return items == 1 ? pass_kernel_ptr<10, 1>(pass) : pass_kernel_ptr<10, 2>(pass);
+    return items == 1 ? kernel_ptr<8, 1>(block) : kernel_ptr<8, 2>(block);
+  return items == 1 ? kernel_ptr<10, 1>(block) : kernel_ptr<10, 2>(block);
 }
 
 // prefix tables for one virtual-block size: [NPASS][nmem+1]
@@ -377,7 +455,7 @@ int upload_prefix(swg_batch b, unsigned vbsize) {
 
 int launch_stage(swg_batch b, int stage, cudaStream_t st) {
   const LaunchConfig &c = kConfigs[b->config];
-  void *fn = pick_kernel(b->ne, c.items);
+  void *fn = pick_kernel(b->ne, c.items, c.block);
   int nmem = b->nmem;
   const Member *mem = b->d_mem;
   const unsigned *pre = b->d_prefix;
@@ -404,17 +482,10 @@ int launch_stage(swg_batch b, int stage, cudaStream_t st) {
     ++g_launches;
     return SWG_OK;
   }
-  for (int pass = 0; pass < NPASS; ++pass) {
-    const unsigned nvb = b->prefix_h[pass * (nmem + 1) + nmem];
-    if (nvb == 0)
-      continue;
-    void *args[] = {&mem, &nmem, &pre, &stage};
-    cudaError_t err = cudaLaunchKernel(pick_pass_kernel(b->ne, c.items, pass),
-                                       dim3(nvb), dim3(c.block), args, 0, st);
-    if (err != cudaSuccess)
-      return cuda_fail(err, "swg_batch: pass launch");
-    ++g_launches;
-  }
+  for (int pass = 0; pass < NPASS; ++pass)
+    TRY(launch_pass(mem, nmem, pre, b->ne, pass, b->heavy, stage,
+                    b->prefix_h[pass * (nmem + 1) + nmem], c.block, c.items,
+                    st));
   (void)vbsize;
   return SWG_OK;
 }
@@ -529,6 +600,7 @@ extern "C" int swg_batch_create(int nmembers, const swg_model *models,
     M.m = models[m]->mesh->view;
     M.p = models[m]->view;
     M.a = models[m]->aux;
+    b->heavy |= batch_heavy_passes(models[m]);
     batch_pass_units(models[m], M.units, M.aux2_base);
     b->versions.push_back(models[m]->version);
   }

@@ -295,11 +295,6 @@ int build_tables(Group &g, double dt) {
         A.m = md->mesh->view;
         A.p = md->view;
         A.a = ad->tp[b].taux[s];
-        // the last stage's PV sum is taped only by a taped advance; the
-        // batched reversals share one table for both kinds of tape and
-        // recompute it
-        if (s == ns - 1)
-          A.a.S1 = nullptr;
         A.v = ad->av;
         A.w = ad->aw;
         A.io = stage_io(ad, ad->tp[b], s, dt);
@@ -370,6 +365,9 @@ int batched_tape(Group &g, int b, bool out_cur, bool copy_in,
   const int n = g.n(), ns = g.ns;
   if (copy_in)
     TRY(group_copy(g, COPY_X0, b, st));
+  unsigned heavy = 0;
+  for (swg_adjoint ad : g.adjs)
+    heavy |= batch_heavy_passes(ad->model);
   for (swg_adjoint ad : g.adjs)
     TRY(tape_prologue(ad, ad->tp[b], out_cur ? ad->cur : nullptr, st));
   for (int s = 0; s < ns; ++s) {
@@ -378,8 +376,12 @@ int batched_tape(Group &g, int b, bool out_cur, bool copy_in,
       for (swg_adjoint ad : g.adjs)
         TRY(tape_stage_copy(ad, ad->tp[b], s, ad->cur, st));
     TRY(batch_launch_passes(g.d_fwd + (size_t(b) * ns + s) * n, n, g.d_fpre,
-                            g.fpre.data(), g.ne, 2, P_VERTEX,
+                            g.fpre.data(), g.ne, 2, heavy, P_VERTEX,
                             aux_only ? P_AUX2 : P_CELL_FINAL, 0, st));
+    if (aux_only) // the PV sums the final passes would have taped
+      TRY(batch_launch_passes(g.d_fwd + (size_t(b) * ns + s) * n, n, g.d_fpre,
+                              g.fpre.data(), g.ne, 2, heavy, P_PV_SUM,
+                              P_PV_SUM, 0, st));
   }
   return SWG_OK;
 }

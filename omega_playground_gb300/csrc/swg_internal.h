@@ -2,6 +2,7 @@
 #pragma once
 
 #include "../../include/swgpu.h"
+#include "swg_fixed.cuh"
 
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
@@ -42,6 +43,13 @@ extern std::atomic<long long> g_launches;
 
 constexpr int MAXE = 6; // edges per cell (MPASMesh::maxedges)
 
+// A gathered neighbour's index and its level-independent weight in the form
+// of the fixed-point sums (swg_fixed.cuh): one 16-byte load per term.
+struct __align__(16) FxSlot {
+  int idx;
+  Wt w;
+};
+
 // Device views of the K-independent tables derived from the MPAS tables.
 // Per-cell slots beyond nedges_on_cell are padded with coefficient 0 and a
 // valid index, so kernels loop a fixed MAXE times without branches.
@@ -67,6 +75,10 @@ struct MeshView {
   const double *inv_dc, *inv_dv, *inv_dv4; // [E]
   const int *eoe;     // nonzero-weight edges_on_edge [E][ne]
   const double *woe;  // their weights / 4 [E][ne]
+  // eoe and woe as fixed-point terms, and each edge's starting sum
+  // (nullptr: a weight is out of their range, the sums run in FP64)
+  const FxSlot *fxe;     // [E][ne]
+  const long long *fxe0; // [E]
   const double *scale2, *scale4; // [E]
   const double *mask; // edge_mask [E][K], nullptr when all ones
   // diagnostics only
@@ -90,6 +102,8 @@ struct ModelView {
   const double *kd2;      // [C][6] eddy_diff2 * scale2 * ckq
   const double *r4;       // [C][6] -eddy_diff4 * scale4 * ckq
   const double *r4sum;    // [C] sum of r4
+  // neighbour cell and r4 as fixed-point terms (e FX_BAD_EXP: out of range)
+  const FxSlot *r4x;      // [C][6]
   // [C] eddy_diff2 * s - r4sum when mesh_scaling_del2 is s on every edge,
   // else nullptr.  The tracer del2 term is then eddy_diff2 * s times the
   // thickness-weighted Laplacian the del4 term already computes, so it
@@ -124,8 +138,19 @@ template <class T> struct AuxViewT {
   // written only when set (the adjoint's tape): 1/h_vertex [V][K], 1/h
   // [C][K] and the PV-flux sum S1 = sum_j w_j F_j [E][K]
   T *rhv, *rh, *S1;
+  // words of the fixed-point sums (swg_fixed.cuh), for the double
+  // instantiation: of F and F Q in pairs [E][K][2] (G is null then: the sums
+  // are its only readers), of ntr and lap [T][C][K].  Null: those sums run
+  // in FP64.
+  fx_t *FGx, *nx, *lx;
 };
 using AuxView = AuxViewT<double>;
+
+// Whether a model's PV sums (pv) and tracer sums (tr) are fixed-point: it
+// then keeps the words of their operands.
+struct FxUse {
+  bool pv, tr;
+};
 
 enum EpiMode {
   EPI_REPLACE = 0,   // tend = x
@@ -206,6 +231,8 @@ void launch_tendency_dual(const MeshView &m, const ModelView &p,
 void launch_aux(const MeshView &m, const ModelView &p, const AuxView &a,
                 const double *h, const double *vn, const double *tr,
                 cudaStream_t st, const Fork *fk = nullptr);
+// the PV sums a.S1 of the last auxiliary passes' fluxes (the adjoint)
+void launch_pv_sum(const MeshView &m, const AuxView &a, cudaStream_t st);
 // one field of a tendency from the last auxiliary state in `a` and the
 // caller's h / vn (the reference's compute_h_tendency, compute_vn_tendency,
 // compute_tr_tendency): field 0 h, 1 vn, 2 tracers; mode EPI_REPLACE or
@@ -244,6 +271,10 @@ struct swg_mesh_s {
   // host copies of the per-edge scaling (the model scales them)
   std::vector<double> scale2_h, scale4_h, ckq_h, inv_dc_h;
   bool scale2_uniform = false; // mesh_scaling_del2 the same on every edge
+  // a level slice's models sum as the model it was sliced for does (fx), so
+  // that their results agree bit for bit
+  bool fx_given = false;
+  swg::FxUse fx{};
   std::vector<int> ec_h, nec_h; // edges_on_cell (padded), nedges_on_cell
   // host copies of the derived tables (the adjoint builds transposes)
   std::vector<int> ev_h, cv_h, nbc_h, ce_h, ve_h, eoe_h;
@@ -287,3 +318,26 @@ struct swg_stepper_s {
   double graph_dt;
   long long graph_launches;    // kernels per captured step
 };
+
+namespace swg {
+
+// The rule for fixed-point sums (swg_fixed.cuh).  Levels: a warp reads a
+// gathered row of its entity's levels, and one table entry per term for all
+// of them; below FX_MIN_LEVELS levels its lanes belong to many entities, and
+// the 16-byte entries of the PV sums cost more than the FP64 instructions
+// they save.  Tracers: the weights are converted once per cell and level and
+// shared by its tracers; without del4 fewer than FX_MIN_TRACERS do not pay
+// for that.
+constexpr int FX_MIN_LEVELS = 2, FX_MIN_TRACERS = 3;
+inline FxUse fx_use(const swg_mesh_s *mesh, const ModelView &p) {
+  if (p.linear)
+    return {false, false};
+  if (mesh->fx_given)
+    return mesh->fx;
+  const bool levels = mesh->nlayers >= FX_MIN_LEVELS;
+  return {levels && p.do_vn && mesh->view.fxe,
+          levels && p.ntracers > 0 &&
+              (p.tr_del4 || p.ntracers >= FX_MIN_TRACERS)};
+}
+
+} // namespace swg

@@ -40,6 +40,15 @@ namespace {
 
 constexpr int TPB = 256;
 
+// Shape of a kernel without or with fixed-point sums (see HTPB)
+template <bool FX> struct Shape {
+  static constexpr int threads = TPB, aux2_blocks = 0, edge_blocks = 0;
+};
+template <> struct Shape<true> {
+  static constexpr int threads = HTPB, aux2_blocks = HEAVY_AUX2_BLOCKS,
+                       edge_blocks = HEAVY_EDGE_BLOCKS;
+};
+
 // Single-instance kernels: one launch per pass over (entity, level),
 // templated on the value type (double, or Dual for the tangent-linear model).
 template <class T>
@@ -69,20 +78,30 @@ __global__ void __launch_bounds__(TPB)
     pt_edge1<T>(m, p, a, h, vn, i);
 }
 
-template <class T>
-__global__ void __launch_bounds__(TPB)
+// TR4 as in pt_aux2
+template <class T, int TR4>
+__global__ void __launch_bounds__(Shape<TR4 == 2>::threads,
+                                  Shape<TR4 == 2>::aux2_blocks)
     k_aux2(MeshView m, ModelView p, AuxViewT<T> a, unsigned base) {
-  const unsigned i = base + blockIdx.x * TPB + threadIdx.x;
+  const unsigned i = base + blockIdx.x * blockDim.x + threadIdx.x;
   if (i < unsigned(m.nvertices + m.ncells) * unsigned(m.nlayers))
-    pt_aux2<T>(m, p, a, i);
+    pt_aux2<T, TR4>(m, p, a, i);
 }
 
-template <int NE, class T>
-__global__ void __launch_bounds__(TPB)
+template <int NE, class T, bool FX>
+__global__ void __launch_bounds__(Shape<FX>::threads, Shape<FX>::edge_blocks)
     k_edge_final(MeshView m, ModelView p, AuxViewT<T> a, StageArgsT<T> s) {
-  const unsigned i = blockIdx.x * TPB + threadIdx.x;
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < unsigned(m.nedges) * unsigned(m.nlayers))
-    pt_edge_final<NE, T>(m, p, a, s, i);
+    pt_edge_final<NE, T, FX>(m, p, a, s, i);
+}
+
+template <int NE>
+__global__ void __launch_bounds__(HTPB)
+    k_pv_sum(MeshView m, AuxView a) {
+  const unsigned i = blockIdx.x * HTPB + threadIdx.x;
+  if (i < unsigned(m.nedges) * unsigned(m.nlayers))
+    pt_pv_sum<NE>(m, a, i);
 }
 
 template <class T>
@@ -90,7 +109,18 @@ __global__ void __launch_bounds__(TPB)
     k_cell_final(MeshView m, ModelView p, AuxViewT<T> a, StageArgsT<T> s) {
   const unsigned i = blockIdx.x * TPB + threadIdx.x;
   if (i < unsigned(m.ncells) * unsigned(m.nlayers))
-    pt_cell_final<T, std::is_same<T, double>::value>(m, p, a, s, i);
+    pt_cell_final<T, 0, false, std::is_same<T, double>::value>(m, p, a, s, i);
+}
+
+// fixed-point tracer sums; D4 = tracer del4
+template <bool D4>
+__global__ void __launch_bounds__(HTPB, HEAVY_CELL_BLOCKS)
+    k_cell_tracers(MeshView m, ModelView p, AuxView a, StageArgs s) {
+  __shared__ fx_t sm[2 * TR_SLOTS * HTPB];
+  const unsigned i = blockIdx.x * HTPB + threadIdx.x;
+  if (i < unsigned(m.ncells) * unsigned(m.nlayers))
+    pt_cell_final<double, D4 ? 2 : 1, true>(m, p, a, s, i, sm + threadIdx.x,
+                                            HTPB);
 }
 
 template <int NE, class T>
@@ -123,7 +153,7 @@ __global__ void __launch_bounds__(TPB)
   const double F = a.mh[i] * vn[i];
   a.F[i] = F;
   if (G)
-    a.G[i] = F * a.Q[i];
+    store_pv(a, i, F, a.Q[i]);
 }
 
 // Elementwise helpers for the unfused stepper path (forcing hook set).
@@ -188,7 +218,64 @@ __global__ void __launch_bounds__(TPB)
     partials[blockIdx.x] = red[0];
 }
 
-unsigned nblocks(long long n) { return unsigned((n + TPB - 1) / TPB); }
+unsigned nblocks(long long n, int tpb = TPB) {
+  return unsigned((n + tpb - 1) / tpb);
+}
+
+template <class T>
+void launch_aux2(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
+                 cudaStream_t st) {
+  const long long K = m.nlayers, VK = m.nvertices * K;
+  // vertex threads only when the velocity del4 curl is needed
+  const unsigned base = (p.do_vn && p.vel_del4) ? 0u : unsigned(VK);
+  const long long n = VK + m.ncells * K - base;
+  if (!(p.ntracers > 0 && p.tr_del4)) {
+    k_aux2<T, 0><<<nblocks(n), TPB, 0, st>>>(m, p, a, base);
+    return;
+  }
+  if constexpr (std::is_same<T, double>::value)
+    if (a.lx) {
+      k_aux2<T, 2><<<nblocks(n, HTPB), HTPB, 0, st>>>(m, p, a, base);
+      return;
+    }
+  k_aux2<T, 1><<<nblocks(n), TPB, 0, st>>>(m, p, a, base);
+}
+
+template <class T>
+void launch_edge_final(const MeshView &m, const ModelView &p,
+                       const AuxViewT<T> &a, const StageArgsT<T> &s,
+                       cudaStream_t st) {
+  const long long n = (long long)m.nedges * m.nlayers;
+  if constexpr (std::is_same<T, double>::value)
+    if (a.FGx) {
+      if (m.ne == 8)
+        k_edge_final<8, T, true><<<nblocks(n, HTPB), HTPB, 0, st>>>(m, p, a, s);
+      else
+        k_edge_final<10, T, true>
+            <<<nblocks(n, HTPB), HTPB, 0, st>>>(m, p, a, s);
+      return;
+    }
+  if (m.ne == 8)
+    k_edge_final<8, T, false><<<nblocks(n), TPB, 0, st>>>(m, p, a, s);
+  else
+    k_edge_final<10, T, false><<<nblocks(n), TPB, 0, st>>>(m, p, a, s);
+}
+
+template <class T>
+void launch_cell_final(const MeshView &m, const ModelView &p,
+                       const AuxViewT<T> &a, const StageArgsT<T> &s,
+                       cudaStream_t st) {
+  const long long n = (long long)m.ncells * m.nlayers;
+  if constexpr (std::is_same<T, double>::value)
+    if (p.ntracers > 0 && a.nx) {
+      if (p.tr_del4)
+        k_cell_tracers<true><<<nblocks(n, HTPB), HTPB, 0, st>>>(m, p, a, s);
+      else
+        k_cell_tracers<false><<<nblocks(n, HTPB), HTPB, 0, st>>>(m, p, a, s);
+      return;
+    }
+  k_cell_final<T><<<nblocks(n), TPB, 0, st>>>(m, p, a, s);
+}
 
 // ---- opt-in per-kernel timing: an event pair around every tendency kernel
 struct Timed {
@@ -308,9 +395,7 @@ void launch_aux_t(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
   const bool tr4 = p.ntracers > 0 && p.tr_del4;
   if (p.do_vn || tr4) {
     Scope sc("k_aux2", st);
-    // vertex threads only when the velocity del4 curl is needed
-    const unsigned base = (p.do_vn && p.vel_del4) ? 0u : unsigned(VK);
-    k_aux2<T><<<nblocks(VK + CK - base), TPB, 0, st>>>(m, p, a, base);
+    launch_aux2<T>(m, p, a, st);
   }
 }
 
@@ -359,15 +444,12 @@ void launch_tendency_t(const MeshView &m, const ModelView &p,
   auto run_edge = [&](cudaStream_t q) {
     NvtxRange r("vn_tendency");
     Scope sc("k_edge_final", q);
-    if (m.ne == 8)
-      k_edge_final<8, T><<<nblocks(EK), TPB, 0, q>>>(m, p, a, s);
-    else
-      k_edge_final<10, T><<<nblocks(EK), TPB, 0, q>>>(m, p, a, s);
+    launch_edge_final<T>(m, p, a, s, q);
   };
   auto run_cell = [&](cudaStream_t q) {
     NvtxRange r("h_tendency+tr_tendency");
     Scope sc("k_cell_final", q);
-    k_cell_final<T><<<nblocks(CK), TPB, 0, q>>>(m, p, a, s);
+    launch_cell_final<T>(m, p, a, s, q);
   };
   // The final passes are independent unless the stage updates the state in
   // place (LSRK): there the edge pass reads h, which the cell pass rewrites,
@@ -398,6 +480,15 @@ void launch_aux(const MeshView &m, const ModelView &p, const AuxView &a,
                 const double *h, const double *vn, const double *tr,
                 cudaStream_t st, const Fork *fk) {
   launch_aux_t<double>(m, p, a, h, vn, tr, st, fk);
+}
+
+void launch_pv_sum(const MeshView &m, const AuxView &a, cudaStream_t st) {
+  const long long n = (long long)m.nedges * m.nlayers;
+  if (m.ne == 8)
+    k_pv_sum<8><<<nblocks(n, HTPB), HTPB, 0, st>>>(m, a);
+  else
+    k_pv_sum<10><<<nblocks(n, HTPB), HTPB, 0, st>>>(m, a);
+  ++g_launches;
 }
 
 void launch_field_tendency(const MeshView &m, const ModelView &p,
@@ -436,10 +527,7 @@ void launch_field_tendency(const MeshView &m, const ModelView &p,
     s.fvn.tend = tend;
     NvtxRange r("vn_tendency");
     Scope sc("k_edge_final", st);
-    if (m.ne == 8)
-      k_edge_final<8, double><<<nblocks(EK), TPB, 0, st>>>(m, q, a, s);
-    else
-      k_edge_final<10, double><<<nblocks(EK), TPB, 0, st>>>(m, q, a, s);
+    launch_edge_final<double>(m, q, a, s, st);
     return;
   }
   // the cell pass writes h when do_h is set and the tracers when ntracers
@@ -453,7 +541,7 @@ void launch_field_tendency(const MeshView &m, const ModelView &p,
   }
   NvtxRange r(field == 0 ? "h_tendency" : "tr_tendency");
   Scope sc("k_cell_final", st);
-  k_cell_final<double><<<nblocks(CK), TPB, 0, st>>>(m, q, a, s);
+  launch_cell_final<double>(m, q, a, s, st);
 }
 
 int fork_create(Fork &f) {

@@ -121,7 +121,7 @@ __global__ void k_noalloc_tables(MeshView m, double f0, double grav,
                                  double kappa4, double *f_vertex, double *gidc,
                                  double *c2e, double *c4e, double *kd2,
                                  double *r4, double *r4sum, double *r4f,
-                                 double *c4i, double *c4v) {
+                                 double *c4i, double *c4v, FxSlot *r4x) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i < m.nvertices)
     f_vertex[i] = f0;
@@ -141,6 +141,8 @@ __global__ void k_noalloc_tables(MeshView m, double f0, double grav,
       const double r = -(kappa4 * m.scale4[e] * m.ckq[6 * i + j]);
       r4[6 * i + j] = r;
       s += r;
+      if (r4x)
+        r4x[6 * i + j] = FxSlot{m.nbc[6 * i + j], fx_table_weight(r)};
     }
     r4sum[i] = s;
     if (r4f) // uniform del2 scaling: the tracer del2 folded into del4
@@ -161,9 +163,10 @@ struct Carve {
 };
 
 // Lays out the model tables and the intermediates the enabled terms need;
-// with base == nullptr it only measures.
-size_t layout(const swg_mesh_s *mesh, const ModelView &pv, unsigned char *base,
-              double *tab[10], AuxView &a) {
+// with base == nullptr it only measures.  words: also the words and the
+// table of the fixed-point sums.
+size_t layout(const swg_mesh_s *mesh, const ModelView &pv, bool words,
+              unsigned char *base, double *tab[11], AuxView &a) {
   const size_t C = mesh->ncells, E = mesh->nedges, V = mesh->nvertices,
                K = mesh->nlayers, T = pv.ntracers;
   Carve cv{base};
@@ -181,6 +184,7 @@ size_t layout(const swg_mesh_s *mesh, const ModelView &pv, unsigned char *base,
   const bool vdiss = vn && (pv.vel_del2 || pv.vel_del4);
   const bool v4 = vn && pv.vel_del4;
   const bool trd = T > 0 && (pv.tr_del2 || pv.tr_del4);
+  const FxUse fx = words ? fx_use(mesh, pv) : FxUse{};
   a = AuxView{};
   if (vn) a.q = cv.take(V * K);
   if (vdiss) a.zeta = cv.take(V * K);
@@ -191,12 +195,22 @@ size_t layout(const swg_mesh_s *mesh, const ModelView &pv, unsigned char *base,
   if (T > 0) a.ntr = cv.take(T * C * K);
   if (T > 0 && pv.tr_del4) a.lap = cv.take(T * C * K);
   a.F = cv.take(E * K);
-  if (vn) a.G = cv.take(E * K);
+  if (vn && !fx.pv) a.G = cv.take(E * K);
   if (vn) a.Q = cv.take(E * K);
   if (trd) a.mh = cv.take(E * K);
   if (vn) a.u2 = cv.take(E * K);
   if (vdiss) a.d2u = cv.take(E * K);
   a.d2u4 = (v4 && mesh->view.dv4_differs) ? cv.take(E * K) : a.d2u;
+  tab[10] = nullptr; // r4x
+  if (fx.tr && pv.tr_del4)
+    tab[10] = cv.take(6 * C * (sizeof(FxSlot) / sizeof(double)));
+  if (fx.pv)
+    a.FGx = reinterpret_cast<fx_t *>(cv.take(2 * E * K));
+  if (fx.tr) {
+    a.nx = reinterpret_cast<fx_t *>(cv.take(T * C * K));
+    if (pv.tr_del4)
+      a.lx = reinterpret_cast<fx_t *>(cv.take(T * C * K));
+  }
   return cv.used;
 }
 
@@ -225,9 +239,13 @@ extern "C" int swg_compute_tendency_noalloc(swg_mesh mesh,
   pv.tr_del4 = params->eddy_diff4 > 0;
   pv.do_h = !params->disable_h_tendency;
   pv.do_vn = !params->disable_vn_tendency;
-  double *tab[10];
+  double *tab[11];
   AuxView a;
-  const size_t need = layout(mesh, pv, nullptr, tab, a);
+  // the words only speed the sums up: a set that fits the array without
+  // them alone runs its sums in FP64
+  const bool words =
+      layout(mesh, pv, true, nullptr, tab, a) <= kScratchBytes;
+  const size_t need = layout(mesh, pv, words, nullptr, tab, a);
   if (need > kScratchBytes) {
     char msg[200];
     std::snprintf(msg, sizeof msg,
@@ -247,7 +265,7 @@ extern "C" int swg_compute_tendency_noalloc(swg_mesh mesh,
                              "above 63");
   unsigned char *base = nullptr;
   TRY(scratch_address(dev, &base));
-  layout(mesh, pv, base, tab, a);
+  layout(mesh, pv, words, base, tab, a);
   pv.f_vertex = tab[0];
   pv.gidc = tab[1];
   pv.c2e = tab[2];
@@ -260,6 +278,8 @@ extern "C" int swg_compute_tendency_noalloc(swg_mesh mesh,
   pv.r4f = fold ? tab[7] : nullptr;
   pv.c4i = tab[8];
   pv.c4v = tab[9];
+  FxSlot *r4x = reinterpret_cast<FxSlot *>(tab[10]);
+  pv.r4x = r4x;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const MeshView &m = mesh->view;
   const long long n = std::max<long long>(
@@ -267,7 +287,7 @@ extern "C" int swg_compute_tendency_noalloc(swg_mesh mesh,
   k_noalloc_tables<<<unsigned((n + 255) / 256), 256, 0, st>>>(
       m, params->f0, params->grav, params->visc_del2, params->visc_del4,
       params->eddy_diff2, params->eddy_diff4, tab[0], tab[1], tab[2], tab[3],
-      tab[4], tab[5], tab[6], fold ? tab[7] : nullptr, tab[8], tab[9]);
+      tab[4], tab[5], tab[6], fold ? tab[7] : nullptr, tab[8], tab[9], r4x);
   ++g_launches;
   StageArgs s{};
   s.h = h;

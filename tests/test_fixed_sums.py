@@ -1,0 +1,166 @@
+"""The fixed-point stencil sums (csrc/swg_fixed.cuh) on the CPU, where the
+header's functions compile as plain C++: words and weights are exact, and a
+sum of N products is within its stated distance of the exact one, over mixed
+magnitudes, signs and cancelling terms; what cannot be represented is
+flagged."""
+import ctypes
+import math
+import os
+import random
+import struct
+import subprocess
+from fractions import Fraction
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(__file__), "..", "omega_playground_gb300",
+                    "csrc")
+SRC = r"""
+#include "swg_fixed.cuh"
+using namespace swg;
+template <int N>
+static double sum(const double *w, const double *x, unsigned *flag) {
+  Wt W[N];
+  fx_t X[N];
+  long long s = 0;
+  unsigned f = 0;
+  for (int j = 0; j < N; ++j) {
+    W[j] = fx_weight(w[j], f);
+    X[j] = fx_word(x[j]);
+    s += W[j].hi;
+  }
+  double r = fx_sum(W, X, fx_start(s), f);
+  *flag = f;
+  return r;
+}
+extern "C" {
+unsigned long long word(double x) { return fx_word(x); }
+void weight(double w, long long *W, int *e, unsigned *flag) {
+  *flag = 0;
+  Wt t = fx_weight(w, *flag);
+  *W = ((long long)t.hi << 28) + t.lo;
+  *e = t.e;
+}
+double sum7(const double *w, const double *x, unsigned *f) { return sum<7>(w, x, f); }
+double sum8(const double *w, const double *x, unsigned *f) { return sum<8>(w, x, f); }
+double sum14(const double *w, const double *x, unsigned *f) { return sum<14>(w, x, f); }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    d = tmp_path_factory.mktemp("fx")
+    src, so = d / "fx.cpp", d / "fx.so"
+    src.write_text(SRC)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC,
+                    "-o", str(so), str(src)], check=True)
+    lib = ctypes.CDLL(str(so))
+    lib.word.restype = ctypes.c_uint64
+    lib.word.argtypes = [ctypes.c_double]
+    lib.weight.argtypes = [ctypes.c_double, ctypes.POINTER(ctypes.c_int64),
+                           ctypes.POINTER(ctypes.c_int),
+                           ctypes.POINTER(ctypes.c_uint)]
+    for n in (7, 8, 14):
+        f = getattr(lib, f"sum{n}")
+        f.restype = ctypes.c_double
+        f.argtypes = [ctypes.POINTER(ctypes.c_double),
+                      ctypes.POINTER(ctypes.c_double),
+                      ctypes.POINTER(ctypes.c_uint)]
+    return lib
+
+
+def _sum(lib, w, x):
+    n = len(w)
+    f = ctypes.c_uint()
+    r = getattr(lib, f"sum{n}")((ctypes.c_double * n)(*w),
+                                (ctypes.c_double * n)(*x), ctypes.byref(f))
+    return r, f.value
+
+
+EDGES = [1.0, -1.0, 1.5, -2.0, 2.0 - 2.0**-52, -(2.0 - 2.0**-52),
+         2.0**-314, -(2.0**-314), 2.0**66, (2.0 - 2.0**-52) * 2.0**66]
+
+
+def test_words_and_weights_are_exact(lib):
+    rng = random.Random(1)
+    xs = EDGES + [rng.choice((-1, 1)) * (1 + rng.random()) * 2.0**rng.randint(-314, 66)
+                  for _ in range(3000)]
+    for x in xs:
+        w = lib.word(x)
+        q = w & 0xff
+        X = struct.unpack("<q", struct.pack("<Q", w & ~0xff))[0]
+        assert 1 <= q <= 127 and 2**60 <= abs(X) < 2**63
+        assert Fraction(X) * Fraction(2)**(3 * q - 377) == Fraction(x)
+        W, e, f = ctypes.c_int64(), ctypes.c_int(), ctypes.c_uint()
+        lib.weight(x, W, e, f)
+        assert f.value == 0 and 2**55 <= abs(W.value) < 2**56
+        assert Fraction(W.value) * Fraction(2)**e.value == Fraction(x)
+    assert lib.word(0.0) == 0 and lib.word(-0.0) == 0
+
+
+def test_what_cannot_be_represented_is_flagged(lib):
+    one = [1.0] * 7
+    for bad in (math.inf, -math.inf, math.nan, 2.0**67, 2.0**-315, 5e-324,
+                -1.7e308):
+        assert lib.word(bad) & 0x80
+        for j in range(7):
+            x = list(one)
+            x[j] = bad
+            assert _sum(lib, one, x)[1] & 0x80
+    for bad in (math.inf, math.nan, 2.0**402, 2.0**-401, 5e-324):
+        w = list(one)
+        w[3] = bad
+        assert _sum(lib, w, one)[1] & 0x80
+    assert _sum(lib, [0.0] * 7, one) == (0.0, 0)
+    assert _sum(lib, one, [0.0] * 7) == (0.0, 0)
+    assert _sum(lib, [0.0, 1.0] + [0.0] * 5, [3.0] * 7) == (3.0, 0)
+
+
+def test_a_sum_of_zero_products_is_zero(lib):
+    rng = random.Random(9)
+    for _ in range(500):
+        w = [rng.uniform(-1, 1) for _ in range(7)]
+        assert _sum(lib, w, [0.0] * 7) == (0.0, 0)
+        x = [rng.uniform(-1, 1) for _ in range(7)]
+        for j in range(7):  # every product has one zero factor
+            (w if rng.random() < 0.5 else x)[j] = 0.0
+        assert _sum(lib, w, x) == (0.0, 0)
+
+
+@pytest.mark.parametrize("n", [7, 8, 14])
+@pytest.mark.parametrize("spread_w,spread_x", [(0, 0), (3, 3), (30, 30),
+                                               (60, 5), (5, 60), (300, 150)])
+def test_sum_error(lib, n, spread_w, spread_x):
+    """|sum - exact| <= n (2^-56 + 2^-59) M + 2^-56 M + 2^-53 |sum|, with M the
+    largest |w_j x_j|: the dropped partial products and shifts, and the two
+    roundings (fixed point, then to double)."""
+    rng = random.Random(1000 * n + 7 * spread_w + spread_x)
+
+    def val(s):
+        return rng.choice((-1, 1)) * (1 + rng.random()) * 2.0**rng.randint(-s, 0)
+
+    for trial in range(1500):
+        w = [val(spread_w) for _ in range(n)]
+        x = [val(spread_x) for _ in range(n)]
+        kind = trial % 5
+        if kind == 1:    # a difference: the last weight cancels the others
+            w[-1] = -math.fsum(w[:-1])
+            x = [1.0 + 1e-6 * v for v in x]
+        elif kind == 2:  # zeros among the values and the weights
+            x[rng.randrange(n)] = 0.0
+            w[rng.randrange(n)] = 0.0
+        elif kind == 3:  # extreme mantissas
+            x = [math.copysign((2 - 2.0**-52) * 2.0**rng.randint(-2, 2), v)
+                 for v in x]
+            w = [math.copysign(2 - 2.0**-52, v) for v in w]
+        elif kind == 4:  # the largest weight meets the smallest value
+            w.sort(key=abs)
+            x.sort(key=abs, reverse=True)
+        r, flag = _sum(lib, w, x)
+        assert flag == 0
+        prods = [Fraction(a) * Fraction(b) for a, b in zip(w, x)]
+        exact, M = sum(prods), max(abs(p) for p in prods)
+        tol = (n * (Fraction(1, 2**56) + Fraction(1, 2**59))
+               + Fraction(1, 2**56)) * M + Fraction(1, 2**53) * abs(exact)
+        assert abs(Fraction(r) - exact) <= tol * Fraction(1001, 1000)
