@@ -168,16 +168,6 @@ pa_vel(const MeshView &m, const ModelView &p, const AuxView &a,
 // branches, and the taped path then issued their FP64 instructions with
 // the predicate off, occupying the FP64 pipe for nothing.
 
-// the forward's Newton reciprocal of x
-__device__ __forceinline__ double fwd_rcp(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  double e = fma(-x, r, 1.0);
-  r = fma(r, e, r);
-  e = fma(-x, r, 1.0);
-  return fma(r, e, r);
-}
-
 static __device__ __noinline__ double mean_h_of(const MeshView &m, const double *h,
                                          int e, int k) {
   const int K = m.nlayers;
@@ -195,7 +185,7 @@ __device__ __forceinline__ double mean_h(const MeshView &m, const AuxView &a,
 
 // 1/h of cell-level i, as the forward's cell pass forms it
 static __device__ __noinline__ double cell_rcp(const double *h, unsigned i) {
-  return fwd_rcp(h[i]);
+  return rcp_nr(h[i]);
 }
 
 // 1/h_vertex of vertex vx, level k, as the forward's vertex pass forms it
@@ -206,7 +196,7 @@ static __device__ __noinline__ double vertex_rcp(const MeshView &m, const double
   for (int j = 1; j < 3; ++j)
     hv = fma(__ldg(m.kvh + 3 * vx + j),
              h[size_t(__ldg(m.cv + 3 * vx + j)) * K + k], hv);
-  return fwd_rcp(hv);
+  return rcp_nr(hv);
 }
 
 // --- pass 2: tracer tendency transposed to the normalised tracers (partial)

@@ -127,6 +127,46 @@ int edge_terms_table(std::vector<void *> &allocs, MeshView &mv, int ne) {
   }
   return SWG_OK;
 }
+__global__ void k_raw_terms(const int *idx, const double *w, long long n,
+                            FxSlot *out, unsigned *bad) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= n)
+    return;
+  unsigned flag = 0;
+  out[i] = FxSlot{idx[i], fx_raw_weight(w[i], flag)};
+  if (flag)
+    atomicOr(bad, flag);
+}
+// mv.cvx, kvx, cdx: left null when a weight is out of range
+int raw_terms_tables(std::vector<void *> &allocs, MeshView &mv) {
+  const long long V3 = 3LL * mv.nvertices, C6 = 6LL * mv.ncells;
+  struct {
+    const int *idx;
+    const double *w;
+    long long n;
+    const FxSlot **out;
+  } tab[] = {{mv.ev, mv.cvr, V3, &mv.cvx},
+             {mv.cv, mv.kvh, V3, &mv.kvx},
+             {mv.ec, mv.ccd, C6, &mv.cdx}};
+  double *b = nullptr;
+  TRY(dalloc(allocs, 1, &b));
+  unsigned *bad = reinterpret_cast<unsigned *>(b), bad_h = 0;
+  FxSlot *slots[3];
+  for (int t = 0; t < 3; ++t) {
+    double *d = nullptr;
+    TRY(dalloc(allocs, size_t(tab[t].n) * (sizeof(FxSlot) / 8), &d));
+    slots[t] = reinterpret_cast<FxSlot *>(d);
+    k_raw_terms<<<unsigned((tab[t].n + 255) / 256), 256>>>(
+        tab[t].idx, tab[t].w, tab[t].n, slots[t], bad);
+    TRY(check_launch("raw terms table"));
+  }
+  cudaError_t err = cudaMemcpy(&bad_h, bad, 4, cudaMemcpyDeviceToHost);
+  if (err != cudaSuccess)
+    return cuda_fail(err, "raw terms table");
+  for (int t = 0; t < 3 && !bad_h; ++t)
+    *tab[t].out = slots[t];
+  return SWG_OK;
+}
 int cell_terms_table(std::vector<void *> &allocs, const MeshView &m,
                      ModelView &pv) {
   double *t = nullptr;
@@ -395,6 +435,7 @@ extern "C" int swg_mesh_create(const swg_mesh_desc *d, swg_mesh *out) try {
       (rc = upload(A, eoe.data(), size_t(NE) * E, &mv.eoe)) ||
       (rc = upload(A, woe.data(), size_t(NE) * E, &mv.woe)) ||
       (rc = edge_terms_table(A, mv, NE)) ||
+      (rc = raw_terms_tables(A, mv)) ||
       (rc = upload(A, m->scale2_h.data(), E, &mv.scale2)) ||
       (rc = upload(A, m->scale4_h.data(), E, &mv.scale4)) ||
       (rc = upload(A, d->area_cell, C, &mv.area_cell_d)) ||
@@ -637,6 +678,7 @@ extern "C" int swg_model_create_ex(swg_mesh mesh, const swg_params *p,
   const bool vdiss = vn && (pv.vel_del2 || pv.vel_del4);
   const bool v4 = vn && pv.vel_del4;
   const FxUse fx = fx_use(mesh, pv);
+  pv.raw = fx.raw;
   if ((rc = alloc_words(A, fx.pv ? E * K : 0, fx.tr ? T * C * K : 0,
                         pv.tr_del4, mesh->fx_given, a)) != SWG_OK) {
     swg_model_destroy(md);

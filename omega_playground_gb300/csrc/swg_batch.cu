@@ -140,7 +140,8 @@ __device__ __forceinline__ int member_of(const unsigned *pre, int nmem,
 // the pass fixed at compile time: each pass kernel is compiled on its own,
 // so a light pass does not carry the registers of the heaviest one and
 // keeps the occupancy of the single-instance kernels.
-template <int NE, int ITEMS, int PASS>
+// RAW: as in entity_sum.
+template <int NE, int ITEMS, int PASS, int RAW>
 __global__ void __launch_bounds__(512)
     k_batch_pass(const Member *__restrict__ mem, int nmem,
                  const unsigned *__restrict__ prefix, int stage) {
@@ -158,7 +159,12 @@ __global__ void __launch_bounds__(512)
       if (i >= n)
         continue;
       // no member keeps the words of the heavy passes' fixed-point sums
-      if (PASS == P_AUX2)
+      const StageArgs &s = M.stage[stage];
+      if (PASS == P_VERTEX)
+        pt_vertex<double, RAW>(M.m, M.p, M.a, s.h, s.vn, i);
+      else if (PASS == P_CELL1)
+        pt_cell1<double, RAW>(M.m, M.p, M.a, s.h, s.vn, s.tr, i);
+      else if (PASS == P_AUX2)
         pt_aux2<double, -2>(M.m, M.p, M.a, M.aux2_base + i);
       else if (PASS == P_EDGE_FINAL)
         pt_edge_final<NE, double, 0>(M.m, M.p, M.a, M.stage[stage], i);
@@ -207,21 +213,28 @@ __global__ void __launch_bounds__(HTPB, heavy_blocks<PASS>())
   }
 }
 
-template <int NE, int ITEMS> void *light_kernel(int pass) {
+template <int NE, int ITEMS, int RAW> void *light_kernel(int pass) {
   switch (pass) {
   case P_VERTEX:
-    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_VERTEX>);
+    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_VERTEX, RAW>);
   case P_CELL1:
-    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_CELL1>);
+    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_CELL1, RAW>);
   case P_EDGE1:
-    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_EDGE1>);
+    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_EDGE1, 0>);
   case P_AUX2:
-    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_AUX2>);
+    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_AUX2, 0>);
   case P_EDGE_FINAL:
-    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_EDGE_FINAL>);
+    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_EDGE_FINAL, 0>);
   default:
-    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_CELL_FINAL>);
+    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_CELL_FINAL, 0>);
   }
+}
+template <int NE, int ITEMS> void *light_kernel(int pass, unsigned heavy) {
+  if (!(heavy & HEAVY_RAW))
+    return light_kernel<NE, ITEMS, 0>(pass);
+  if (heavy & HEAVY_NO_RAW) // members of both kinds
+    return light_kernel<NE, ITEMS, -1>(pass);
+  return light_kernel<NE, ITEMS, 1>(pass);
 }
 template <int NE> void *heavy_kernel(int pass) {
   switch (pass) {
@@ -239,7 +252,10 @@ template <int NE> void *heavy_kernel(int pass) {
 unsigned batch_heavy_passes(const swg_model_s *md) {
   const AuxView &a = md->aux;
   return (a.lx ? 1u << P_AUX2 : 0u) | (a.FGx ? 1u << P_EDGE_FINAL : 0u) |
-         (a.nx ? 1u << P_CELL_FINAL : 0u) | 1u << P_PV_SUM;
+         (a.nx ? 1u << P_CELL_FINAL : 0u) | 1u << P_PV_SUM |
+         (md->view.raw & RAW_DIV ? HEAVY_RAW
+          : md->view.raw         ? HEAVY_RAW | HEAVY_NO_RAW
+                                 : HEAVY_NO_RAW);
 }
 
 // One pass over nvb virtual blocks of block x items elements (block a power
@@ -258,9 +274,11 @@ static int launch_pass(const Member *mem, int nmem, const unsigned *prefix,
     nvb <<= shift;
     block = HTPB;
   } else if (items == 2) {
-    fn = ne == 8 ? light_kernel<8, 2>(pass) : light_kernel<10, 2>(pass);
+    fn = ne == 8 ? light_kernel<8, 2>(pass, heavy)
+                 : light_kernel<10, 2>(pass, heavy);
   } else {
-    fn = ne == 8 ? light_kernel<8, 1>(pass) : light_kernel<10, 1>(pass);
+    fn = ne == 8 ? light_kernel<8, 1>(pass, heavy)
+                 : light_kernel<10, 1>(pass, heavy);
   }
   void *args[] = {&mem, &nmem, &prefix, &stage, &shift};
   cudaError_t err = cudaLaunchKernel(fn, dim3(nvb), dim3(block), args, 0, st);

@@ -52,8 +52,10 @@ __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(
 __device__ __forceinline__ Dual mul_rn(double a, Dual b) { return a * b; }
 __device__ __forceinline__ Dual add_rn(Dual a, Dual b) { return a + b; }
 
-// 1/x: hardware estimate refined by two Newton-Raphson steps
-// r <- r + r (1 - x r); each step squares the relative error of the estimate.
+// 1/x: hardware estimate r refined by one third-order step: with the residual
+// e = 1 - x r, 1/x = r / (1 - e) = r (1 + e + e^2 + ...), so r + r (e + e^2)
+// has the relative error e^3 (the estimate's cubed) before its one rounding.
+// Three FP64 instructions; two Newton steps take four.
 // The estimate is the .ftz form: a subnormal input (|x| < 2^-1022) counts as
 // zero (result infinite) and a result below 2^-1022 flushes to zero, so the
 // function is for |x| in [2^-1022, 2^1022], far beyond any thickness.  On
@@ -62,15 +64,36 @@ __device__ __forceinline__ Dual add_rn(Dual a, Dual b) { return a + b; }
 __device__ __forceinline__ double rcp_nr(double x) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  double e = fma(-x, r, 1.0);
-  r = fma(r, e, r);
-  e = fma(-x, r, 1.0);
-  return fma(r, e, r);
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
 }
 __device__ __forceinline__ Dual rcp_nr(Dual x) {
   const double r = rcp_nr(x.v);
   return {r, -(r * r) * x.d};
 }
+
+// x / 2 and 2 x through the exponent field (exact, as the products are): an
+// integer addition instead of an FP64 instruction.  Zeros, subnormals, the
+// ends of the range, infinities and NaN take the product, out of line so that
+// it is not issued with the predicate off.
+static __device__ __noinline__ double times_rare(double x, double c) {
+  return c * x;
+}
+__device__ __forceinline__ double half_of(double x) {
+  const int hi = __double2hiint(x);
+  if ((unsigned(hi) & 0x7ff00000u) - 0x00200000u > 0x7fc00000u)
+    return times_rare(x, 0.5);
+  return __hiloint2double(hi - 0x00100000, __double2loint(x));
+}
+__device__ __forceinline__ double twice(double x) {
+  const int hi = __double2hiint(x);
+  if ((unsigned(hi) & 0x7ff00000u) - 0x00100000u > 0x7fc00000u)
+    return times_rare(x, 2.0);
+  return __hiloint2double(hi + 0x00100000, __double2loint(x));
+}
+__device__ __forceinline__ Dual half_of(Dual x) { return 0.5 * x; }
+__device__ __forceinline__ Dual twice(Dual x) { return 2.0 * x; }
+
 using ::sqrt;
 __device__ __forceinline__ Dual sqrt(Dual x) {
   const double s = ::sqrt(x.v);
@@ -177,25 +200,64 @@ __device__ __forceinline__ void epilogue(const Epilogue &ep,
   }
 }
 
+// ---- sums of doubles over an entity's neighbours, fixed-point
+//
+// One entity's terms from a table: N slots from `tab`, the field x.
+template <int N>
+__device__ __forceinline__ double raw_sum(const FxSlot *tab, const double *x,
+                                          unsigned K, unsigned k, bool &slow) {
+  Wt w[N];
+  double v[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const int4 t = __ldg(reinterpret_cast<const int4 *>(tab) + j);
+    w[j] = {t.y, t.z, t.w};
+    v[j] = x[unsigned(t.x) * K + k];
+  }
+  return fx_raw_sum(w, v, slow);
+}
+// the same in FP64, for terms the fixed-point sum leaves to it (out of line:
+// see times_rare)
+static __device__ __noinline__ double dot_f64(const double *coef,
+                                              const int *idx, int n,
+                                              const double *x, int K, int k) {
+  double t = __ldg(coef) * x[size_t(__ldg(idx)) * K + k];
+  for (int j = 1; j < n; ++j)
+    t = fma(__ldg(coef + j), x[size_t(__ldg(idx + j)) * K + k], t);
+  return t;
+}
+// sum_j coef_j x_(idx_j) over the N terms of entity c: RAW fixed-point from
+// the table tab (1), in FP64 (0), or as the model's RAW_* bit BIT says (-1)
+template <int N, int RAW, int BIT, class T>
+__device__ __forceinline__ T entity_sum(const ModelView &p, const FxSlot *tab,
+                                        const double *coef, const int *idx,
+                                        int c, const T *x, int K, int k) {
+  if constexpr (std::is_same<T, double>::value && RAW != 0) {
+    if (RAW == 1 || (p.raw & BIT)) {
+      bool slow = false;
+      double t = raw_sum<N>(tab + N * c, x, unsigned(K), unsigned(k), slow);
+      if (slow)
+        t = dot_f64(coef + N * c, idx + N * c, N, x, K, k);
+      return t;
+    }
+  }
+  T t = __ldg(coef + N * c) * x[size_t(__ldg(idx + N * c)) * K + k];
+#pragma unroll
+  for (int j = 1; j < N; ++j)
+    t = fma(__ldg(coef + N * c + j), x[size_t(__ldg(idx + N * c + j)) * K + k],
+            t);
+  return t;
+}
+
 // Vertex pass: relative vorticity and (rvort + f) / h_vertex.
-template <class T>
+template <class T, int RAW = -1>
 __device__ __forceinline__ void
 pt_vertex(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
           const T *__restrict__ h, const T *__restrict__ vn, unsigned i) {
   const int K = m.nlayers;
   const int v = int(i / unsigned(K)), k = int(i - unsigned(v) * unsigned(K));
-  T z, hv;
-  {
-    const int e = __ldg(m.ev + 3 * v), c = __ldg(m.cv + 3 * v);
-    z = __ldg(m.cvr + 3 * v) * vn[size_t(e) * K + k];
-    hv = __ldg(m.kvh + 3 * v) * h[size_t(c) * K + k];
-  }
-#pragma unroll
-  for (int j = 1; j < 3; ++j) {
-    const int e = __ldg(m.ev + 3 * v + j), c = __ldg(m.cv + 3 * v + j);
-    z = fma(__ldg(m.cvr + 3 * v + j), vn[size_t(e) * K + k], z);
-    hv = fma(__ldg(m.kvh + 3 * v + j), h[size_t(c) * K + k], hv);
-  }
+  const T hv = entity_sum<3, RAW, RAW_VERTEX>(p, m.kvx, m.kvh, m.cv, v, h, K, k);
+  const T z = entity_sum<3, RAW, RAW_VERTEX>(p, m.cvx, m.cvr, m.ev, v, vn, K, k);
   const T r = rcp_nr(hv);
   a.q[i] = (z + __ldg(p.f_vertex + v)) * r;
   if (a.rhv)
@@ -206,7 +268,7 @@ pt_vertex(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
 
 // Cell pass 1: velocity divergence (for the dissipation terms) and the
 // normalised tracers tr / h.
-template <class T>
+template <class T, int RAW = -1>
 __device__ __forceinline__ void
 pt_cell1(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
          const T *__restrict__ h, const T *__restrict__ vn,
@@ -215,12 +277,7 @@ pt_cell1(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
   const unsigned CK = unsigned(m.ncells) * unsigned(K);
   const int c = int(i / unsigned(K)), k = int(i - unsigned(c) * unsigned(K));
   if (p.do_vn && (p.vel_del2 | p.vel_del4)) {
-    T dv = __ldg(m.ccd + 6 * c) * vn[size_t(__ldg(m.ec + 6 * c)) * K + k];
-#pragma unroll
-    for (int j = 1; j < MAXE; ++j)
-      dv = fma(__ldg(m.ccd + 6 * c + j),
-               vn[size_t(__ldg(m.ec + 6 * c + j)) * K + k], dv);
-    a.div[i] = dv;
+    a.div[i] = entity_sum<MAXE, RAW, RAW_DIV>(p, m.cdx, m.ccd, m.ec, c, vn, K, k);
   }
   if (p.ntracers > 0) {
     const T r = rcp_nr(h[i]);
@@ -260,7 +317,7 @@ pt_edge1(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
   const int K = m.nlayers;
   const int e = int(i / unsigned(K)), k = int(i - unsigned(e) * unsigned(K));
   const int c0 = __ldg(m.ce + 2 * e), c1 = __ldg(m.ce + 2 * e + 1);
-  const T mh = 0.5 * (h[size_t(c0) * K + k] + h[size_t(c1) * K + k]);
+  const T mh = half_of(h[size_t(c0) * K + k] + h[size_t(c1) * K + k]);
   const T u = vn[i];
   const T F = mh * u;
   a.F[i] = F;
@@ -404,12 +461,7 @@ __device__ __forceinline__ void pt_aux2(const MeshView &m, const ModelView &p,
     if (!vel)
       return;
     const int v = int(i / unsigned(K)), k = int(i - unsigned(v) * unsigned(K));
-    T z = __ldg(m.cvr + 3 * v) * a.d2u4[size_t(__ldg(m.ev + 3 * v)) * K + k];
-#pragma unroll
-    for (int j = 1; j < 3; ++j)
-      z = fma(__ldg(m.cvr + 3 * v + j),
-              a.d2u4[size_t(__ldg(m.ev + 3 * v + j)) * K + k], z);
-    a.z4[i] = z;
+    a.z4[i] = entity_sum<3, 0, 0>(p, nullptr, m.cvr, m.ev, v, a.d2u4, K, k);
     return;
   }
   i -= VK;
@@ -419,21 +471,10 @@ __device__ __forceinline__ void pt_aux2(const MeshView &m, const ModelView &p,
   const bool tr4 = TR4 < 0 ? p.ntracers > 0 && p.tr_del4 : TR4 != 0;
   if (p.do_vn) {
     // ke = sum_j dv dc / (4 area) vn_j^2
-    T ke = __ldg(m.cke + 6 * c) * a.u2[size_t(__ldg(m.ec + 6 * c)) * K + k];
-#pragma unroll
-    for (int j = 1; j < MAXE; ++j)
-      ke = fma(__ldg(m.cke + 6 * c + j),
-               a.u2[size_t(__ldg(m.ec + 6 * c + j)) * K + k], ke);
-    a.ke[i] = ke;
+    a.ke[i] = entity_sum<MAXE, 0, 0>(p, nullptr, m.cke, m.ec, c, a.u2, K, k);
   }
-  if (vel) {
-    T d = __ldg(m.ccd + 6 * c) * a.d2u4[size_t(__ldg(m.ec + 6 * c)) * K + k];
-#pragma unroll
-    for (int j = 1; j < MAXE; ++j)
-      d = fma(__ldg(m.ccd + 6 * c + j),
-              a.d2u4[size_t(__ldg(m.ec + 6 * c + j)) * K + k], d);
-    a.d4[i] = d;
-  }
+  if (vel)
+    a.d4[i] = entity_sum<MAXE, 0, 0>(p, nullptr, m.ccd, m.ec, c, a.d2u4, K, k);
   if (tr4) {
     // L = sum_j w_j (n_nb - n_c), w_j = ckq_j mean_h_j
     T w[MAXE], M;
@@ -930,7 +971,7 @@ pt_cell_final(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
       Sa = add_rn(Sa, w[j]);
   }
   if (p.do_h) // -sum_j ccd_j F_j, or nothing with thickness advection off
-    epilogue(s.ep, s.fh, i, p.off_hadv ? T{} : 2.0 * Sa, hin);
+    epilogue(s.ep, s.fh, i, p.off_hadv ? T{} : twice(Sa), hin);
   if (p.ntracers == 0)
     return;
   if (p.off_tr_hadv) { // tracer advection off: only diffusion weights
@@ -1034,7 +1075,10 @@ struct Member {
 // (swg_batch.cu) element counts of a model's passes
 void batch_pass_units(const swg_model_s *md, unsigned units[NPASS],
                       unsigned &aux2_base);
-// (swg_batch.cu) the passes a model runs with fixed-point sums, as a bit set
+// (swg_batch.cu) the passes a model runs with sums of words, as a bit set, and
+// whether all or none of its sums of doubles are fixed-point (of a batch: in
+// some member; both bits: the passes look at each member)
+constexpr unsigned HEAVY_RAW = 1u << 16, HEAVY_NO_RAW = 1u << 17;
 unsigned batch_heavy_passes(const swg_model_s *md);
 // (swg_batch.cu) passes [pass0, pass1] of stage `stage` over the nmem
 // members of the device table `mem`, one 256-thread block per virtual block

@@ -220,4 +220,75 @@ SWG_HD double fx_sum(const Wt (&w)[N], const fx_t (&x)[N], long long start,
   return fx_finish(a, P);
 }
 
+// ---- sums of float64 values as they are
+//
+// The same sums from the bits of the doubles, for values gathered too few
+// times to be worth a word: about 20 integer instructions per term.
+// X = mantissa 2^8 (2^60 <= |X| < 2^61), a negative one's complement instead
+// of its negation (2^-60 of it).  Weights carry their exponent as
+// (e - 65) 2^20, so that adding the double's exponent field gives the
+// product's; magnitudes 2^-120 .. 2^120.  A largest product outside
+// 2^-760 .. 2^770 or so (all terms zero, infinities, NaN, subnormals among
+// them) makes the caller evaluate the sum in FP64.
+constexpr int FXR_ZERO = -0x7fffffff - 1;
+SWG_HD Wt fx_raw_weight(double w, unsigned &flag) {
+  Wt r = fx_weight(w, flag);
+  if (r.e == FX_ZERO_EXP) {
+    r.e = FXR_ZERO;
+  } else {
+    if (r.e < -175 || r.e > 65)
+      flag |= FX_FLAG;
+    r.e = (r.e - 65) * (1 << 20);
+  }
+  return r;
+}
+
+// sum_j w_j x_j; sets `slow` when it has to be evaluated in FP64
+template <int N>
+SWG_HD double fx_raw_sum(const Wt (&w)[N], const double (&x)[N], bool &slow) {
+  static_assert(N <= 7, "the sum of hi in 32 bits");
+  int p[N], P = FXR_ZERO, sum = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    p[j] = int(unsigned(fx_bits(x[j]) >> 32) & 0x7ff00000u) + w[j].e;
+    P = P > p[j] ? P : p[j];
+    sum += w[j].hi;
+  }
+  FxAcc a{0, 0, fx_start(sum)};
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const fx_t b = fx_bits(x[j]);
+    const unsigned s = (unsigned(P) - unsigned(p[j])) >> 20;
+    fx_t X = ((b & 0xfffffffffffffULL) | 0x10000000000000ULL) << 8;
+#ifdef __CUDA_ARCH__
+    asm("shr.u64 %0, %0, %1;" : "+l"(X) : "r"(s));
+#else
+    X = s > 63 ? 0 : X >> s;
+#endif
+    const unsigned sgn = unsigned(int(unsigned(b >> 32)) >> 31);
+    const int xh = int(unsigned(X >> 32) ^ sgn);
+    const int xl = int(unsigned(X) ^ sgn ^ 0x80000000u);
+    fx_mad(a.hh, w[j].hi, xh);
+    fx_mad(a.m1, w[j].hi, xl);
+    fx_mad(a.m2, w[j].lo, xh);
+  }
+  slow = slow || unsigned(P) - (200u << 20) >= (1535u << 20);
+  const long long t = a.m2 + (a.m1 >> 4);
+  const long long R = a.hh + (t >> 28);
+#ifdef __CUDA_ARCH__
+  const double d = __ll2double_rn(R);
+  const int hi = __double2hiint(d);
+  return __hiloint2double(hi == 0 ? 0 : hi + (P - (958 << 20)),
+                          __double2loint(d));
+#else
+  const double d = double(R);
+  fx_t b = fx_bits(d);
+  if (b)
+    b += fx_t((long long)(P - (958 << 20))) << 32;
+  double r;
+  std::memcpy(&r, &b, 8);
+  return r;
+#endif
+}
+
 } // namespace swg

@@ -197,7 +197,8 @@ static int make_chunk(swg_host_stepper hs, int kind, int nstages, Chunk &c) {
   swg_model src = hs->model;
   TRY(mesh_slice(src->mesh, c.k0, c.kc, &c.mesh));
   c.mesh->fx_given = true;
-  c.mesh->fx = {src->aux.FGx != nullptr, src->aux.nx != nullptr};
+  c.mesh->fx = {src->aux.FGx != nullptr, src->aux.nx != nullptr,
+                src->view.raw};
   swg_model_options o{};
   o.linear = src->view.linear;
   o.h0 = src->view.h0;

@@ -79,6 +79,9 @@ struct MeshView {
   // (nullptr: a weight is out of their range, the sums run in FP64)
   const FxSlot *fxe;     // [E][ne]
   const long long *fxe0; // [E]
+  // cvr and kvh with their edges and cells [V][3] and ccd with its edges
+  // [C][6], as terms of the sums of doubles (fx_raw_sum; null: out of range)
+  const FxSlot *cvx, *kvx, *cdx;
   const double *scale2, *scale4; // [E]
   const double *mask; // edge_mask [E][K], nullptr when all ones
   // diagnostics only
@@ -88,6 +91,9 @@ struct MeshView {
   const int *maxlev_c;       // [C] levels summed per cell, nullptr = nlayers
   const int *maxlev_v;       // [V] levels summed per vertex, nullptr = nlayers
 };
+
+constexpr int RAW_VERTEX = 1; // vorticity and vertex thickness
+constexpr int RAW_DIV = 2;    // velocity divergence
 
 // Parameters and parameter-scaled coefficient tables of one model.
 struct ModelView {
@@ -114,6 +120,8 @@ struct ModelView {
   // LinearShallowWaterModel (mean thickness h0; f4 = 4 f0, the Coriolis
   // factor for the weights/4 table), and the optional bottom drag
   int linear, drag;
+  // RAW_* bits: sums of doubles that are fixed-point
+  int raw;
   int drag_level; // the level of the model's arrays that carries the drag
   double h0, f4, drag_coeff;
   // tendency terms switched off after create (the reference's m_enabled
@@ -146,10 +154,12 @@ template <class T> struct AuxViewT {
 };
 using AuxView = AuxViewT<double>;
 
-// Whether a model's PV sums (pv) and tracer sums (tr) are fixed-point: it
-// then keeps the words of their operands.
+// Whether a model's PV sums (pv) and tracer sums (tr) are fixed-point (it
+// then keeps the words of their operands), and which of its sums of doubles
+// are (raw, RAW_* bits).
 struct FxUse {
   bool pv, tr;
+  int raw;
 };
 
 enum EpiMode {
@@ -325,19 +335,33 @@ namespace swg {
 // gathered row of its entity's levels, and one table entry per term for all
 // of them; below FX_MIN_LEVELS levels its lanes belong to many entities, and
 // the 16-byte entries of the PV sums cost more than the FP64 instructions
-// they save.  Tracers: the weights are converted once per cell and level and
+// they save (edge pass, 65536 cells: 1 level 16.3 us in FP64, 18.7 fixed; 2
+// levels 17.7 and 16.2; 4 levels 22.4 and 18.7).  Size: the edge pass keeps
+// 24 warps per SM resident, 117k threads; a model with fewer edge-levels does
+// not fill them, and the longer chain of a sum shows (RK4 step, 1 tracer, 48x48
+// cells x 16 levels: 77.5 us in FP64, 80.2 fixed; 64x64x16: 120.6 and 114.4).
+// Tracers: the weights are converted once per cell and level and
 // shared by its tracers; without del4 fewer than FX_MIN_TRACERS do not pay
 // for that.
 constexpr int FX_MIN_LEVELS = 2, FX_MIN_TRACERS = 3;
+constexpr long long FX_MIN_EDGE_LEVELS = 1 << 17;
+// with more tracers the first cell pass is bound by their memory traffic, not
+// by the divergence's FP64 (8 tracers, 256x256x64: 149 us in FP64, 154 fixed)
+constexpr int FX_MAX_DIV_TRACERS = 4;
 inline FxUse fx_use(const swg_mesh_s *mesh, const ModelView &p) {
   if (p.linear)
-    return {false, false};
+    return {false, false, 0};
   if (mesh->fx_given)
     return mesh->fx;
   const bool levels = mesh->nlayers >= FX_MIN_LEVELS;
-  return {levels && p.do_vn && mesh->view.fxe,
+  const bool large =
+      levels && (long long)mesh->nedges * mesh->nlayers >= FX_MIN_EDGE_LEVELS;
+  return {large && p.do_vn && mesh->view.fxe,
           levels && p.ntracers > 0 &&
-              (p.tr_del4 || p.ntracers >= FX_MIN_TRACERS)};
+              (p.tr_del4 || p.ntracers >= FX_MIN_TRACERS),
+          !large || !p.do_vn || !mesh->view.cvx ? 0
+          : p.ntracers <= FX_MAX_DIV_TRACERS    ? RAW_VERTEX | RAW_DIV
+                                                : RAW_VERTEX};
 }
 
 } // namespace swg

@@ -280,6 +280,7 @@ extern "C" int swg_compute_tendency_noalloc(swg_mesh mesh,
   pv.c4v = tab[9];
   FxSlot *r4x = reinterpret_cast<FxSlot *>(tab[10]);
   pv.r4x = r4x;
+  pv.raw = fx_use(mesh, pv).raw;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const MeshView &m = mesh->view;
   const long long n = std::max<long long>(

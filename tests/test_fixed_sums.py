@@ -33,7 +33,23 @@ static double sum(const double *w, const double *x, unsigned *flag) {
   *flag = f;
   return r;
 }
+template <int N>
+static double raw(const double *w, const double *x, unsigned *slow) {
+  Wt W[N];
+  double X[N];
+  unsigned f = 0;
+  for (int j = 0; j < N; ++j) {
+    W[j] = fx_raw_weight(w[j], f);
+    X[j] = x[j];
+  }
+  bool s = f != 0;
+  double r = fx_raw_sum(W, X, s);
+  *slow = s;
+  return r;
+}
 extern "C" {
+double raw3(const double *w, const double *x, unsigned *f) { return raw<3>(w, x, f); }
+double raw6(const double *w, const double *x, unsigned *f) { return raw<6>(w, x, f); }
 unsigned long long word(double x) { return fx_word(x); }
 void weight(double w, long long *W, int *e, unsigned *flag) {
   *flag = 0;
@@ -61,8 +77,8 @@ def lib(tmp_path_factory):
     lib.weight.argtypes = [ctypes.c_double, ctypes.POINTER(ctypes.c_int64),
                            ctypes.POINTER(ctypes.c_int),
                            ctypes.POINTER(ctypes.c_uint)]
-    for n in (7, 8, 14):
-        f = getattr(lib, f"sum{n}")
+    for f in [getattr(lib, f"sum{n}") for n in (7, 8, 14)] + [lib.raw3,
+                                                              lib.raw6]:
         f.restype = ctypes.c_double
         f.argtypes = [ctypes.POINTER(ctypes.c_double),
                       ctypes.POINTER(ctypes.c_double),
@@ -164,3 +180,63 @@ def test_sum_error(lib, n, spread_w, spread_x):
         tol = (n * (Fraction(1, 2**56) + Fraction(1, 2**59))
                + Fraction(1, 2**56)) * M + Fraction(1, 2**53) * abs(exact)
         assert abs(Fraction(r) - exact) <= tol * Fraction(1001, 1000)
+
+
+def _raw(lib, w, x):
+    n = len(w)
+    f = ctypes.c_uint()
+    r = (lib.raw3 if n == 3 else lib.raw6)(
+        (ctypes.c_double * n)(*w), (ctypes.c_double * n)(*x), ctypes.byref(f))
+    return r, f.value
+
+
+@pytest.mark.parametrize("n", [3, 6])
+@pytest.mark.parametrize("spread_w,spread_x", [(0, 0), (3, 3), (30, 30),
+                                               (60, 5), (5, 60), (100, 400)])
+def test_raw_sum_error(lib, n, spread_w, spread_x):
+    """As the sums of words, with one more 2^-60 of each negative term (its
+    complement for its negation) and with values that keep 2^60 <= |X|."""
+    rng = random.Random(77 * n + 7 * spread_w + spread_x)
+
+    def val(s):
+        return rng.choice((-1, 1)) * (1 + rng.random()) * 2.0**rng.randint(-s, 0)
+
+    for trial in range(2000):
+        w = [val(spread_w) for _ in range(n)]
+        x = [val(spread_x) for _ in range(n)]
+        kind = trial % 4
+        if kind == 1:
+            w[-1] = -math.fsum(w[:-1])
+            x = [1.0 + 1e-6 * v for v in x]
+        elif kind == 2:
+            x[rng.randrange(n)] = rng.choice((0.0, -0.0))
+            w[rng.randrange(n)] = 0.0
+        elif kind == 3:
+            x = [math.copysign((2 - 2.0**-52) * 2.0**rng.randint(-2, 2), v)
+                 for v in x]
+            w = [math.copysign(2 - 2.0**-52, v) for v in w]
+        prods = [Fraction(a) * Fraction(b) for a, b in zip(w, x)]
+        exact, M = sum(prods), max(abs(p) for p in prods)
+        r, slow = _raw(lib, w, x)
+        if M == 0 or abs(w[-1]) < 2.0**-120:
+            continue
+        assert not slow
+        tol = (n * (Fraction(1, 2**56) + Fraction(1, 2**59)
+                    + Fraction(1, 2**59))
+               + Fraction(1, 2**56)) * M + Fraction(1, 2**53) * abs(exact)
+        assert abs(Fraction(r) - exact) <= tol * Fraction(1001, 1000)
+
+
+def test_raw_sum_leaves_the_rest_to_fp64(lib):
+    one = [1.0] * 6
+    for bad in (math.inf, -math.inf, math.nan, 1e300):
+        for j in range(6):
+            x = list(one)
+            x[j] = bad
+            assert _raw(lib, one, x)[1]
+    for x in ([0.0] * 6, [-0.0] * 6, [5e-324] * 6, [1e-290] * 6):
+        assert _raw(lib, one, x)[1]
+    assert _raw(lib, [2.0**121] + [1.0] * 5, one)[1]
+    assert _raw(lib, [2.0**-121] + [1.0] * 5, one)[1]
+    assert _raw(lib, [0.0, 0.0, 2.0], [math.pi, 1.0, 3.0]) == (6.0, 0)
+    assert _raw(lib, [1.0] * 3, [0.0, -0.0, 3.0]) == (3.0, 0)
