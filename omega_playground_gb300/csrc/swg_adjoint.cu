@@ -395,7 +395,8 @@ int alloc_tape(swg_adjoint ad, int b, int s) {
   if (md->view.do_vn) {
     TRY(zal(A, V * K, &t.rhv));
     // the last stage's PV sum comes from the step's final passes (a taped
-    // advance) or, where they do not run, from a pass of its own
+    // advance) or, where they do not run, from a pass of its own (fixed-point
+    // sums) or from the adjoint's edge pass (adjoint_step's last_s1)
     TRY(zal(A, E * K, &t.S1));
   }
   if (md->params.ntracers > 0)
@@ -490,12 +491,13 @@ void adj_tendency(swg_adjoint ad, const double *h, const double *vn,
                   cudaStream_t st) {
   swg_model md = ad->model;
   launch_aux(md->mesh->view, md->view, md->aux, h, vn, tr, st, &md->fork);
-  // the PV sums go to the edge pass's own work array: each thread reads its
-  // S1 before it writes that element of lQ
+  // fixed-point PV sums go to the edge pass's own work array: each thread
+  // reads its S1 before it writes that element of lQ
   AuxView aux = md->aux;
-  aux.S1 = ad->aw.lQ;
-  if (md->view.do_vn && !md->view.off_pv)
+  if (aux.FGx && !md->view.off_pv) {
+    aux.S1 = ad->aw.lQ;
     launch_pv_sum(md->mesh->view, aux, st);
+  }
   AdjIO io{};
   io.h = h;
   io.vn = vn;
@@ -535,7 +537,7 @@ int tape_step(swg_adjoint ad, TapeSlot &tp, double dt, swg_state out,
       const double *h, *vn, *tr;
       stage_ptrs(ad, tp, s, &h, &vn, &tr);
       launch_aux(md->mesh->view, pv, tp.taux[s], h, vn, tr, st, &md->fork);
-      if (pv.do_vn && !pv.off_pv)
+      if (tp.taux[s].FGx && !pv.off_pv)
         launch_pv_sum(md->mesh->view, tp.taux[s], st);
       continue;
     }
@@ -561,14 +563,20 @@ int tape_step(swg_adjoint ad, TapeSlot &tp, double dt, swg_state out,
 // lamX_s = lamX_{s+1} + J(X_s)^T mu_s and
 // mu_{s-1} = dt b_{s-1} lamX_s + a_s mu_s; the step's adjoint is lamX_0.
 // The output passes accumulate lamX in lacc and form mu_{s-1} from it.
-int adjoint_step(swg_adjoint ad, const TapeSlot &tp, double dt,
+// last_s1: the tape was written by a taped advance, whose last stage ran
+// its final passes and taped that stage's PV sum too (without it, only
+// fixed-point sums are there)
+int adjoint_step(swg_adjoint ad, const TapeSlot &tp, double dt, bool last_s1,
                  cudaStream_t st) {
   const int ns = ad->ns;
   if (ns % 2 != 0)
     lincomb(ad->mu, ad->lam, nullptr, dt * step_rkb(ad)[ns - 1], 0.0,
             (long long)words(ad->model), st);
   for (int s = ns - 1; s >= 0; --s) {
-    adj_passes(ad, tp.taux[s], stage_io(ad, tp, s, dt), st);
+    AuxView aux = tp.taux[s];
+    if (s == ns - 1 && !last_s1 && !aux.FGx)
+      aux.S1 = nullptr;
+    adj_passes(ad, aux, stage_io(ad, tp, s, dt), st);
   }
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? SWG_OK : cuda_fail(err, "swg_adjoint: adjoint step");
@@ -854,12 +862,12 @@ int run_action(swg_adjoint ad, const AdjAction &a, cudaStream_t st, bool two) {
     // forcing), replayed from a graph captured on first use
     rc = replay(ad, tp.tape_adj, st, [&](cudaStream_t cs) {
       TRY(tape_step(ad, tp, ad->dt, nullptr, cs));
-      return adjoint_step(ad, tp, ad->dt, cs);
+      return adjoint_step(ad, tp, ad->dt, false, cs);
     });
   } else {
     // a reversal without its own tape follows a taped advance into tp
     rc = replay(ad, tp.adj, st, [&](cudaStream_t cs) {
-      return adjoint_step(ad, tp, ad->dt, cs);
+      return adjoint_step(ad, tp, ad->dt, true, cs);
     });
   }
   if (rc == SWG_OK && two && (e = cudaEventRecord(tp.free_ev, st)) != cudaSuccess)

@@ -199,6 +199,19 @@ static __device__ __noinline__ double vertex_rcp(const MeshView &m, const double
   return rcp_nr(hv);
 }
 
+// the PV flux sum S1 = sum_j w_j F_j of edge e, level k, in FP64 (a model with
+// fixed-point sums has it in S1: pt_pv_sum)
+template <int NE>
+__device__ __noinline__ double s1_of(const MeshView &m, const AuxView &a,
+                                     int e, int k) {
+  const int K = m.nlayers;
+  double S1 = 0;
+  for (int j = 0; j < NE; ++j)
+    S1 = fma(__ldg(m.woe + NE * e + j),
+             a.F[size_t(__ldg(m.eoe + NE * e + j)) * K + k], S1);
+  return S1;
+}
+
 // --- pass 2: tracer tendency transposed to the normalised tracers (partial)
 // and to the tracer Laplacian.  D2, D4: tracer del2 / del4 on, as
 // compile-time switches (with runtime flags the diffusion arrays stayed in
@@ -321,7 +334,7 @@ pa_edge(const MeshView &m, const ModelView &p, const AuxView &a,
         lFq = fma(ws, w.Qmu[is], lFq);
       }
       // (S1 may be lQ itself, see adj_tendency)
-      const double S1 = a.S1[i];
+      const double S1 = a.S1 ? a.S1[i] : s1_of<NE>(m, a, e, k);
       w.lQ[i] = fma(S1, mu, F * lG);
       lF = fma(a.Q[i], lG, lFq);
     } else {

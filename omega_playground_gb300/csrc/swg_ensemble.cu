@@ -295,6 +295,11 @@ int build_tables(Group &g, double dt) {
         A.m = md->mesh->view;
         A.p = md->view;
         A.a = ad->tp[b].taux[s];
+        // the last stage's PV sum is taped only by a taped advance; the
+        // batched reversals share one table for both kinds of tape and
+        // recompute it, unless it is fixed-point: then batched_tape sees to it
+        if (s == ns - 1 && !A.a.FGx)
+          A.a.S1 = nullptr;
         A.v = ad->av;
         A.w = ad->aw;
         A.io = stage_io(ad, ad->tp[b], s, dt);
@@ -378,7 +383,8 @@ int batched_tape(Group &g, int b, bool out_cur, bool copy_in,
     TRY(batch_launch_passes(g.d_fwd + (size_t(b) * ns + s) * n, n, g.d_fpre,
                             g.fpre.data(), g.ne, 2, heavy, P_VERTEX,
                             aux_only ? P_AUX2 : P_CELL_FINAL, 0, st));
-    if (aux_only) // the PV sums the final passes would have taped
+    // the fixed-point PV sums the final passes would have taped
+    if (aux_only && (heavy >> P_EDGE_FINAL & 1))
       TRY(batch_launch_passes(g.d_fwd + (size_t(b) * ns + s) * n, n, g.d_fpre,
                               g.fpre.data(), g.ne, 2, heavy, P_PV_SUM,
                               P_PV_SUM, 0, st));

@@ -345,6 +345,11 @@ namespace swg {
 // for that.
 constexpr int FX_MIN_LEVELS = 2, FX_MIN_TRACERS = 3;
 constexpr long long FX_MIN_EDGE_LEVELS = 1 << 17;
+// Below this a stage's two pairs of independent passes are one launch each
+// (RK4 step, all terms, 2 tracers, replayed from a graph: 26x26 cells x 32
+// levels, 65k edge-levels, 88.0 us apart and 75.9 together; 40x40x16, 77k:
+// 90.2 and 91.9, the joint kernels' registers being those of the cell pass).
+constexpr long long SMALL_EDGE_LEVELS = 1 << 16;
 // with more tracers the first cell pass is bound by their memory traffic, not
 // by the divergence's FP64 (8 tracers, 256x256x64: 149 us in FP64, 154 fixed)
 constexpr int FX_MAX_DIV_TRACERS = 4;

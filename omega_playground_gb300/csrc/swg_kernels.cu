@@ -144,6 +144,41 @@ __global__ void __launch_bounds__(TPB)
     pt_lin_cell<T>(m, p, s, i);
 }
 
+// Small models (below SMALL_EDGE_LEVELS): the two independent pairs of passes
+// as one launch each, so a stage is a chain of four launches without the
+// fork and join of the pairs (four events).  A launch of such a model takes
+// its latency, about 3 us, whatever its passes compute (RK4 step of 12x10
+// cells, 3 levels, 2 tracers, launched one by one: 114 us forked, 94 joint).
+__global__ void __launch_bounds__(HTPB)
+    k_vertex_cell1(MeshView m, ModelView p, AuxView a,
+                   const double *__restrict__ h, const double *__restrict__ vn,
+                   const double *__restrict__ tr) {
+  const unsigned VK = unsigned(m.nvertices) * unsigned(m.nlayers);
+  const unsigned i = blockIdx.x * HTPB + threadIdx.x;
+  if (i < VK)
+    pt_vertex<double, 0>(m, p, a, h, vn, i);
+  else if (i - VK < unsigned(m.ncells) * unsigned(m.nlayers))
+    pt_cell1<double, 0>(m, p, a, h, vn, tr, i - VK);
+}
+// blocks below `edge_blocks` take edges, the others cells (not for an
+// in-place stage, whose edges read the h that the cells rewrite)
+template <int NE>
+__global__ void __launch_bounds__(HTPB, HEAVY_CELL_BLOCKS)
+    k_final(MeshView m, ModelView p, AuxView a, StageArgs s,
+            unsigned edge_blocks) {
+  __shared__ fx_t sm[2 * TR_SLOTS * HTPB];
+  if (blockIdx.x < edge_blocks) {
+    const unsigned i = blockIdx.x * HTPB + threadIdx.x;
+    if (i < unsigned(m.nedges) * unsigned(m.nlayers))
+      pt_edge_final<NE, double, 0>(m, p, a, s, i);
+  } else {
+    const unsigned i = (blockIdx.x - edge_blocks) * HTPB + threadIdx.x;
+    if (i < unsigned(m.ncells) * unsigned(m.nlayers))
+      pt_cell_final<double, -1, true, true>(m, p, a, s, i, sm + threadIdx.x,
+                                            HTPB);
+  }
+}
+
 // Thickness flux of a per-field tendency call (compute_h/vn/tr_tendency):
 // F = mean_h vn from the last auxiliary state's mean thickness and the
 // caller's normal velocity (pv_flux_edge.hpp and thickness_hadv_cell.hpp
@@ -362,6 +397,14 @@ int profile_read(int max_kernels, char *names, double *total_ms,
 
 namespace {
 
+// Whether the pairs of passes run as one launch (per-kernel timing keeps them
+// apart).
+template <class T> bool small_model(const MeshView &m, const AuxViewT<T> &a) {
+  if (!std::is_same<T, double>::value || g_profile)
+    return false;
+  return !a.FGx && (long long)m.nedges * m.nlayers < SMALL_EDGE_LEVELS;
+}
+
 template <class T>
 void launch_aux_t(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
                   const T *h, const T *vn, const T *tr, cudaStream_t st,
@@ -393,7 +436,13 @@ void launch_aux_t(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
   // that each event pair times its own kernel alone
   if (g_profile)
     fk = nullptr;
-  if (vert && cell1)
+  if (vert && cell1 && small_model<T>(m, a)) {
+    if constexpr (std::is_same<T, double>::value) {
+      Scope sc("k_vertex_cell1", st);
+      k_vertex_cell1<<<nblocks(VK + CK, HTPB), HTPB, 0, st>>>(m, p, a, h, vn,
+                                                              tr);
+    }
+  } else if (vert && cell1)
     fork_join(fk, st, run_vertex, run_cell1);
   else if (vert)
     run_vertex(st);
@@ -465,7 +514,17 @@ void launch_tendency_t(const MeshView &m, const ModelView &p,
   // The final passes are independent unless the stage updates the state in
   // place (LSRK): there the edge pass reads h, which the cell pass rewrites,
   // so the edge pass goes first.
-  if (edge && cell)
+  if (edge && cell && s.ep.mode != EPI_LSRK && small_model<T>(m, a)) {
+    if constexpr (std::is_same<T, double>::value) {
+      NvtxRange r("vn_tendency+h_tendency+tr_tendency");
+      Scope sc("k_final", st);
+      const unsigned nb = nblocks(EK, HTPB);
+      if (m.ne == 8)
+        k_final<8><<<nb + nblocks(CK, HTPB), HTPB, 0, st>>>(m, p, a, s, nb);
+      else
+        k_final<10><<<nb + nblocks(CK, HTPB), HTPB, 0, st>>>(m, p, a, s, nb);
+    }
+  } else if (edge && cell)
     fork_join(s.ep.mode == EPI_LSRK || g_profile ? nullptr : fk, st, run_edge,
               run_cell);
   else if (edge)
