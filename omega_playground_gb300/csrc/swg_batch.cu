@@ -140,9 +140,15 @@ __device__ __forceinline__ int member_of(const unsigned *pre, int nmem,
 // the pass fixed at compile time: each pass kernel is compiled on its own,
 // so a light pass does not carry the registers of the heaviest one and
 // keeps the occupancy of the single-instance kernels.
-// RAW: as in entity_sum.
+// RAW: as in entity_sum; for P_AUX2 1 means that no member has a tracer
+// Laplacian in FP64.  The vertex and the first edge pass are held to 32
+// registers, 64 warps per SM (12 members, 2 elements a thread: 86 us with 40
+// and 80 with 32, 155 us with 38 and 141 with 32).
+template <int PASS> constexpr int light_blocks() {
+  return PASS == P_VERTEX || PASS == P_EDGE1 ? 4 : 0;
+}
 template <int NE, int ITEMS, int PASS, int RAW>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(512, light_blocks<PASS>())
     k_batch_pass(const Member *__restrict__ mem, int nmem,
                  const unsigned *__restrict__ prefix, int stage) {
   const unsigned vbsize = blockDim.x * ITEMS;
@@ -165,7 +171,7 @@ __global__ void __launch_bounds__(512)
       else if (PASS == P_CELL1)
         pt_cell1<double, RAW>(M.m, M.p, M.a, s.h, s.vn, s.tr, i);
       else if (PASS == P_AUX2)
-        pt_aux2<double, -2>(M.m, M.p, M.a, M.aux2_base + i);
+        pt_aux2<double, RAW == 1 ? 0 : -2>(M.m, M.p, M.a, M.aux2_base + i);
       else if (PASS == P_EDGE_FINAL)
         pt_edge_final<NE, double, 0>(M.m, M.p, M.a, M.stage[stage], i);
       else if (PASS == P_CELL_FINAL)
@@ -222,7 +228,7 @@ template <int NE, int ITEMS, int RAW> void *light_kernel(int pass) {
   case P_EDGE1:
     return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_EDGE1, 0>);
   case P_AUX2:
-    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_AUX2, 0>);
+    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_AUX2, RAW == 1>);
   case P_EDGE_FINAL:
     return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_EDGE_FINAL, 0>);
   default:
@@ -230,6 +236,9 @@ template <int NE, int ITEMS, int RAW> void *light_kernel(int pass) {
   }
 }
 template <int NE, int ITEMS> void *light_kernel(int pass, unsigned heavy) {
+  if (pass == P_AUX2)
+    return heavy & HEAVY_LAP ? light_kernel<NE, ITEMS, 0>(pass)
+                             : light_kernel<NE, ITEMS, 1>(pass);
   if (!(heavy & HEAVY_RAW))
     return light_kernel<NE, ITEMS, 0>(pass);
   if (heavy & HEAVY_NO_RAW) // members of both kinds
@@ -253,6 +262,7 @@ unsigned batch_heavy_passes(const swg_model_s *md) {
   const AuxView &a = md->aux;
   return (a.lx ? 1u << P_AUX2 : 0u) | (a.FGx ? 1u << P_EDGE_FINAL : 0u) |
          (a.nx ? 1u << P_CELL_FINAL : 0u) | 1u << P_PV_SUM |
+         (a.lap && !a.lx ? HEAVY_LAP : 0u) |
          (md->view.raw & RAW_DIV ? HEAVY_RAW
           : md->view.raw         ? HEAVY_RAW | HEAVY_NO_RAW
                                  : HEAVY_NO_RAW);

@@ -1078,7 +1078,9 @@ void batch_pass_units(const swg_model_s *md, unsigned units[NPASS],
 // (swg_batch.cu) the passes a model runs with sums of words, as a bit set, and
 // whether all or none of its sums of doubles are fixed-point (of a batch: in
 // some member; both bits: the passes look at each member)
-constexpr unsigned HEAVY_RAW = 1u << 16, HEAVY_NO_RAW = 1u << 17;
+// and whether it has tracer Laplacians in FP64
+constexpr unsigned HEAVY_RAW = 1u << 16, HEAVY_NO_RAW = 1u << 17,
+                   HEAVY_LAP = 1u << 18;
 unsigned batch_heavy_passes(const swg_model_s *md);
 // (swg_batch.cu) passes [pass0, pass1] of stage `stage` over the nmem
 // members of the device table `mem`, one 256-thread block per virtual block
