@@ -1,9 +1,10 @@
 // Batched ensembles: many independent instances (uneven mesh size, level
 // count and tracer count) advanced together.
 //
-// One RK stage of every member is one persistent cooperative kernel that
-// runs the six passes of the tendency (swg_device.cuh) over all members,
-// with a grid barrier between passes.  Work is cut into virtual blocks of
+// One RK stage of every member is the six passes of the tendency
+// (swg_device.cuh) over all members: a launch each, or one persistent
+// cooperative kernel with a grid barrier between passes (the passes with
+// fixed-point sums of words are launches of their own in any case).  Work is cut into virtual blocks of
 // blockDim*ITEMS (entity, level) elements; a per-pass prefix table over the
 // members maps a virtual block to its member, and resident blocks stride
 // over the virtual blocks.  The arithmetic per element is exactly the
@@ -85,12 +86,30 @@ __device__ __forceinline__ void run_pass(int pass, const Member &M, int stage,
   }
 }
 
+// the same where no member keeps the words of the pass's fixed-point sums
+template <int NE, int RAW>
+__device__ __forceinline__ void light_pass(int pass, const Member &M, int stage,
+                                           unsigned i) {
+  const StageArgs &s = M.stage[stage];
+  switch (pass) {
+  case P_VERTEX: pt_vertex<double, RAW>(M.m, M.p, M.a, s.h, s.vn, i); break;
+  case P_CELL1:
+    pt_cell1<double, RAW>(M.m, M.p, M.a, s.h, s.vn, s.tr, i);
+    break;
+  case P_EDGE1: pt_edge1(M.m, M.p, M.a, s.h, s.vn, i); break;
+  case P_AUX2: pt_aux2<double, -2>(M.m, M.p, M.a, M.aux2_base + i); break;
+  case P_EDGE_FINAL: pt_edge_final<NE, double, 0>(M.m, M.p, M.a, s, i); break;
+  default: pt_cell_final<double, 0>(M.m, M.p, M.a, s, i); break;
+  }
+}
+
 // Passes [pass0, pass1] of stage `stage` for all members.  prefix[pass] has
-// nmem+1 entries: virtual-block offsets of the members in that pass.
-// BLOCK: threads per block; 24 resident warps per SM (80 registers) where the
-// block allows them.
-template <int NE, int ITEMS, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, BLOCK > 256 ? 1 : 768 / BLOCK)
+// nmem+1 entries: virtual-block offsets of the members in that pass.  Passes
+// with fixed-point sums of words are not its own (launch_stage): with them
+// here every pass ran at their registers (4 members 100x100x40, 256 threads:
+// 2681 us a step, 2309 without).
+template <int NE, int ITEMS>
+__global__ void __launch_bounds__(512)
     k_batch(const Member *__restrict__ mem, int nmem,
             const unsigned *__restrict__ prefix, int stage, int pass0,
             int pass1, BatchSync *bs, long long limit) {
@@ -114,7 +133,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCK > 256 ? 1 : 768 / BLOCK)
       for (int it = 0; it < ITEMS; ++it) {
         const unsigned i = first + it * blockDim.x;
         if (i < n)
-          run_pass<NE>(pass, M, stage, i);
+          light_pass<NE, -1>(pass, M, stage, i);
       }
     }
     if (pass < pass1 && !grid_barrier(bs, limit))
@@ -164,20 +183,10 @@ __global__ void __launch_bounds__(512, light_blocks<PASS>())
       const unsigned i = first + it * blockDim.x;
       if (i >= n)
         continue;
-      // no member keeps the words of the heavy passes' fixed-point sums
-      const StageArgs &s = M.stage[stage];
-      if (PASS == P_VERTEX)
-        pt_vertex<double, RAW>(M.m, M.p, M.a, s.h, s.vn, i);
-      else if (PASS == P_CELL1)
-        pt_cell1<double, RAW>(M.m, M.p, M.a, s.h, s.vn, s.tr, i);
-      else if (PASS == P_AUX2)
-        pt_aux2<double, RAW == 1 ? 0 : -2>(M.m, M.p, M.a, M.aux2_base + i);
-      else if (PASS == P_EDGE_FINAL)
-        pt_edge_final<NE, double, 0>(M.m, M.p, M.a, M.stage[stage], i);
-      else if (PASS == P_CELL_FINAL)
-        pt_cell_final<double, 0>(M.m, M.p, M.a, M.stage[stage], i);
+      if (PASS == P_AUX2 && RAW == 1)
+        pt_aux2<double, 0>(M.m, M.p, M.a, M.aux2_base + i);
       else
-        run_pass<NE>(PASS, M, stage, i);
+        light_pass<NE, RAW>(PASS, M, stage, i);
     }
   }
 }
@@ -185,10 +194,12 @@ __global__ void __launch_bounds__(512, light_blocks<PASS>())
 // The passes with fixed-point sums (P_AUX2, P_EDGE_FINAL, P_CELL_FINAL, and
 // P_PV_SUM) of batches whose members (or some of them) keep the words, in
 // the single-instance kernels' shape whatever the configuration's block:
-// 2^shift blocks of HTPB threads per virtual block, HEAVY_ITEMS elements a
-// thread (finding the member and reading its descriptor is a chain of loads
-// at each block's start).
-constexpr int HEAVY_ITEMS = 2;
+// 2^shift blocks of HTPB threads per virtual block, `items` elements a thread:
+// two, since finding the member and reading its descriptor is a chain of loads
+// at each block's start, but one where no more than HEAVY_WAVE blocks result
+// (10 resident on each SM), whose time is that of one element (3 members up
+// to 8x8x3, 3 tracers: 131 us a step with two, 115 with one).
+constexpr unsigned HEAVY_WAVE = 1520;
 template <int PASS> constexpr int heavy_blocks() {
   return PASS == P_AUX2 ? HEAVY_AUX2_BLOCKS
          : PASS == P_CELL_FINAL ? HEAVY_CELL_BLOCKS
@@ -197,7 +208,8 @@ template <int PASS> constexpr int heavy_blocks() {
 template <int NE, int PASS>
 __global__ void __launch_bounds__(HTPB, heavy_blocks<PASS>())
     k_batch_heavy(const Member *__restrict__ mem, int nmem,
-                  const unsigned *__restrict__ prefix, int stage, int shift) {
+                  const unsigned *__restrict__ prefix, int stage, int shift,
+                  int items) {
   __shared__ fx_t sm[PASS == P_CELL_FINAL ? 2 * TR_SLOTS * HTPB : 1];
   constexpr int DOMAIN = PASS == P_PV_SUM ? P_EDGE_FINAL : PASS;
   const unsigned *pre = prefix + DOMAIN * (nmem + 1);
@@ -205,10 +217,9 @@ __global__ void __launch_bounds__(HTPB, heavy_blocks<PASS>())
   const int lo = member_of(pre, nmem, vb);
   const Member &M = mem[lo];
   const unsigned n = M.units[DOMAIN];
-  unsigned i = (blockIdx.x - (pre[lo] << shift)) * (HTPB * HEAVY_ITEMS) +
-               threadIdx.x;
+  unsigned i = (blockIdx.x - (pre[lo] << shift)) * (HTPB * items) + threadIdx.x;
 #pragma unroll 1
-  for (int it = 0; it < HEAVY_ITEMS && i < n; ++it, i += HTPB) {
+  for (int it = 0; it < items && i < n; ++it, i += HTPB) {
     if (PASS == P_CELL_FINAL)
       pt_cell_final<double, -1, true>(M.m, M.p, M.a, M.stage[stage], i,
                                       sm + threadIdx.x, HTPB);
@@ -279,8 +290,13 @@ static int launch_pass(const Member *mem, int nmem, const unsigned *prefix,
   int shift = 0;
   if (heavy >> pass & 1) {
     fn = ne == 8 ? heavy_kernel<8>(pass) : heavy_kernel<10>(pass);
-    while ((HTPB * HEAVY_ITEMS << shift) < block * items)
-      ++shift;
+    while ((HTPB << shift) < block * items)
+      ++shift; // at least 1
+    items = 1;
+    if (nvb << shift > HEAVY_WAVE) {
+      items = 2;
+      --shift;
+    }
     nvb <<= shift;
     block = HTPB;
   } else if (items == 2) {
@@ -290,7 +306,7 @@ static int launch_pass(const Member *mem, int nmem, const unsigned *prefix,
     fn = ne == 8 ? light_kernel<8, 1>(pass, heavy)
                  : light_kernel<10, 1>(pass, heavy);
   }
-  void *args[] = {&mem, &nmem, &prefix, &stage, &shift};
+  void *args[] = {&mem, &nmem, &prefix, &stage, &shift, &items};
   cudaError_t err = cudaLaunchKernel(fn, dim3(nvb), dim3(block), args, 0, st);
   if (err != cudaSuccess)
     return cuda_fail(err, "batched passes: launch");
@@ -332,6 +348,10 @@ static const LaunchConfig kConfigs[] = {
     {1, 256, 1}, {1, 128, 1}, {1, 512, 1}, {1, 256, 2}, {1, 128, 2},
     {0, 256, 1}, {0, 128, 1}, {0, 512, 1}, {0, 256, 2},
 };
+// a batch's shape until it is tuned or told: a launch per pass, 128 threads
+// (a step of 2 to 12 equal members from 8x8x3 to 100x100x40, 1 to 4 tracers:
+// 101-2040 us, with the persistent 256 threads 131-2309)
+constexpr int DEFAULT_CONFIG = 6;
 static const int kNumConfigs = sizeof(kConfigs) / sizeof(kConfigs[0]);
 
 struct swg_batch_s {
@@ -448,17 +468,12 @@ int upload_members(swg_batch b, double dt) {
   return SWG_OK;
 }
 
-template <int NE, int ITEMS> void *kernel_ptr(int block) {
-  switch (block) {
-  case 128: return reinterpret_cast<void *>(&k_batch<NE, ITEMS, 128>);
-  case 256: return reinterpret_cast<void *>(&k_batch<NE, ITEMS, 256>);
-  default: return reinterpret_cast<void *>(&k_batch<NE, ITEMS, 512>);
-  }
-}
-void *pick_kernel(int ne, int items, int block) {
+void *pick_kernel(int ne, int items) {
   if (ne == 8)
-    return items == 1 ? kernel_ptr<8, 1>(block) : kernel_ptr<8, 2>(block);
-  return items == 1 ? kernel_ptr<10, 1>(block) : kernel_ptr<10, 2>(block);
+    return items == 1 ? reinterpret_cast<void *>(&k_batch<8, 1>)
+                      : reinterpret_cast<void *>(&k_batch<8, 2>);
+  return items == 1 ? reinterpret_cast<void *>(&k_batch<10, 1>)
+                    : reinterpret_cast<void *>(&k_batch<10, 2>);
 }
 
 // prefix tables for one virtual-block size: [NPASS][nmem+1]
@@ -481,40 +496,51 @@ int upload_prefix(swg_batch b, unsigned vbsize) {
   return SWG_OK;
 }
 
-int launch_stage(swg_batch b, int stage, cudaStream_t st) {
+// Passes [p0, p1] of one stage in one cooperative launch
+int launch_persistent(swg_batch b, int stage, int p0, int p1, cudaStream_t st) {
   const LaunchConfig &c = kConfigs[b->config];
-  void *fn = pick_kernel(b->ne, c.items, c.block);
+  void *fn = pick_kernel(b->ne, c.items);
   int nmem = b->nmem;
   const Member *mem = b->d_mem;
   const unsigned *pre = b->d_prefix;
   BatchSync *bs = b->d_sync;
   long long limit = b->limit;
-  const unsigned vbsize = unsigned(c.block * c.items);
-  if (c.persistent) {
-    int per_sm = 0;
-    cudaError_t err =
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, c.block, 0);
-    if (err != cudaSuccess || per_sm < 1)
-      return cuda_fail(err != cudaSuccess ? err : cudaErrorInvalidConfiguration,
-                       "swg_batch: occupancy");
-    // no more resident blocks than the largest pass has virtual blocks
-    unsigned maxvb = 1;
-    for (int pass = 0; pass < NPASS; ++pass)
-      maxvb = std::max(maxvb, b->prefix_h[pass * (nmem + 1) + nmem]);
-    const unsigned grid = std::min<unsigned>(unsigned(per_sm * b->sms), maxvb);
-    int p0 = 0, p1 = NPASS - 1;
-    void *args[] = {&mem, &nmem, &pre, &stage, &p0, &p1, &bs, &limit};
-    err = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(c.block), args, 0, st);
-    if (err != cudaSuccess)
-      return cuda_fail(err, "swg_batch: cooperative launch");
-    ++g_launches;
-    return SWG_OK;
+  int per_sm = 0;
+  cudaError_t err =
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, c.block, 0);
+  if (err != cudaSuccess || per_sm < 1)
+    return cuda_fail(err != cudaSuccess ? err : cudaErrorInvalidConfiguration,
+                     "swg_batch: occupancy");
+  // no more resident blocks than the largest pass has virtual blocks
+  unsigned maxvb = 1;
+  for (int pass = p0; pass <= p1; ++pass)
+    maxvb = std::max(maxvb, b->prefix_h[pass * (nmem + 1) + nmem]);
+  const unsigned grid = std::min<unsigned>(unsigned(per_sm * b->sms), maxvb);
+  void *args[] = {&mem, &nmem, &pre, &stage, &p0, &p1, &bs, &limit};
+  err = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(c.block), args, 0, st);
+  if (err != cudaSuccess)
+    return cuda_fail(err, "swg_batch: cooperative launch");
+  ++g_launches;
+  return SWG_OK;
+}
+
+// A persistent configuration runs the passes that no member has fixed-point
+// sums of words in; the others are launches of their own (k_batch_heavy).
+int launch_stage(swg_batch b, int stage, cudaStream_t st) {
+  const LaunchConfig &c = kConfigs[b->config];
+  for (int pass = 0; pass < NPASS; ++pass) {
+    int last = pass;
+    if (c.persistent && !(b->heavy >> pass & 1)) {
+      while (last + 1 < NPASS && !(b->heavy >> (last + 1) & 1))
+        ++last;
+      TRY(launch_persistent(b, stage, pass, last, st));
+    } else {
+      TRY(launch_pass(b->d_mem, b->nmem, b->d_prefix, b->ne, pass, b->heavy,
+                      stage, b->prefix_h[pass * (b->nmem + 1) + b->nmem],
+                      c.block, c.items, st));
+    }
+    pass = last;
   }
-  for (int pass = 0; pass < NPASS; ++pass)
-    TRY(launch_pass(mem, nmem, pre, b->ne, pass, b->heavy, stage,
-                    b->prefix_h[pass * (nmem + 1) + nmem], c.block, c.items,
-                    st));
-  (void)vbsize;
   return SWG_OK;
 }
 
@@ -655,7 +681,7 @@ extern "C" int swg_batch_create(int nmembers, const swg_model *models,
       rc = cuda_fail(err, "swg_batch_create: device setup");
   }
   if (rc == SWG_OK)
-    rc = set_config(b, 0);
+    rc = set_config(b, DEFAULT_CONFIG);
   if (rc != SWG_OK) {
     swg_batch_destroy(b);
     return rc;
