@@ -163,11 +163,14 @@ __device__ __forceinline__ int member_of(const unsigned *pre, int nmem,
 // Laplacian in FP64.  The vertex and the first edge pass are held to 32
 // registers, 64 warps per SM (12 members, 2 elements a thread: 86 us with 40
 // and 80 with 32, 155 us with 38 and 141 with 32).
-template <int PASS> constexpr int light_blocks() {
-  return PASS == P_VERTEX || PASS == P_EDGE1 ? 4 : 0;
+// FULL: not where 48 warps per SM hold all of the pass's elements: there a
+// thread's loads in flight count (gradients of 3 members 12x8x33, 3 steps:
+// 932 us with it, 901 without).
+template <int PASS, bool FULL> constexpr int light_blocks() {
+  return FULL && (PASS == P_VERTEX || PASS == P_EDGE1) ? 4 : 0;
 }
-template <int NE, int ITEMS, int PASS, int RAW>
-__global__ void __launch_bounds__(512, light_blocks<PASS>())
+template <int NE, int ITEMS, int PASS, int RAW, bool FULL>
+__global__ void __launch_bounds__(512, light_blocks<PASS, FULL>())
     k_batch_pass(const Member *__restrict__ mem, int nmem,
                  const unsigned *__restrict__ prefix, int stage) {
   const unsigned vbsize = blockDim.x * ITEMS;
@@ -200,6 +203,8 @@ __global__ void __launch_bounds__(512, light_blocks<PASS>())
 // (10 resident on each SM), whose time is that of one element (3 members up
 // to 8x8x3, 3 tracers: 131 us a step with two, 115 with one).
 constexpr unsigned HEAVY_WAVE = 1520;
+// threads of 48 warps on each SM
+constexpr unsigned LIGHT_WAVE = 152 * 1536;
 template <int PASS> constexpr int heavy_blocks() {
   return PASS == P_AUX2 ? HEAVY_AUX2_BLOCKS
          : PASS == P_CELL_FINAL ? HEAVY_CELL_BLOCKS
@@ -230,31 +235,47 @@ __global__ void __launch_bounds__(HTPB, heavy_blocks<PASS>())
   }
 }
 
-template <int NE, int ITEMS, int RAW> void *light_kernel(int pass) {
+template <int NE, int ITEMS, int RAW, bool FULL>
+void *light_kernel(int pass) {
   switch (pass) {
   case P_VERTEX:
-    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_VERTEX, RAW>);
+    return reinterpret_cast<void *>(
+        &k_batch_pass<NE, ITEMS, P_VERTEX, RAW, FULL>);
   case P_CELL1:
-    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_CELL1, RAW>);
+    return reinterpret_cast<void *>(
+        &k_batch_pass<NE, ITEMS, P_CELL1, RAW, true>);
   case P_EDGE1:
-    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_EDGE1, 0>);
+    return reinterpret_cast<void *>(
+        &k_batch_pass<NE, ITEMS, P_EDGE1, 0, FULL>);
   case P_AUX2:
-    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_AUX2, RAW == 1>);
+    return reinterpret_cast<void *>(
+        &k_batch_pass<NE, ITEMS, P_AUX2, RAW == 1, true>);
   case P_EDGE_FINAL:
-    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_EDGE_FINAL, 0>);
+    return reinterpret_cast<void *>(
+        &k_batch_pass<NE, ITEMS, P_EDGE_FINAL, 0, true>);
   default:
-    return reinterpret_cast<void *>(&k_batch_pass<NE, ITEMS, P_CELL_FINAL, 0>);
+    return reinterpret_cast<void *>(
+        &k_batch_pass<NE, ITEMS, P_CELL_FINAL, 0, true>);
   }
 }
-template <int NE, int ITEMS> void *light_kernel(int pass, unsigned heavy) {
+template <int NE, int ITEMS, bool FULL>
+void *light_kernel(int pass, unsigned heavy) {
   if (pass == P_AUX2)
-    return heavy & HEAVY_LAP ? light_kernel<NE, ITEMS, 0>(pass)
-                             : light_kernel<NE, ITEMS, 1>(pass);
+    return heavy & HEAVY_LAP || !FULL ? light_kernel<NE, ITEMS, 0, FULL>(pass)
+                                      : light_kernel<NE, ITEMS, 1, FULL>(pass);
   if (!(heavy & HEAVY_RAW))
-    return light_kernel<NE, ITEMS, 0>(pass);
+    return light_kernel<NE, ITEMS, 0, FULL>(pass);
   if (heavy & HEAVY_NO_RAW) // members of both kinds
-    return light_kernel<NE, ITEMS, -1>(pass);
-  return light_kernel<NE, ITEMS, 1>(pass);
+    return light_kernel<NE, ITEMS, -1, FULL>(pass);
+  return light_kernel<NE, ITEMS, 1, FULL>(pass);
+}
+template <int NE>
+void *light_kernel(int pass, unsigned heavy, int items, bool full) {
+  if (items == 2)
+    return full ? light_kernel<NE, 2, true>(pass, heavy)
+                : light_kernel<NE, 2, false>(pass, heavy);
+  return full ? light_kernel<NE, 1, true>(pass, heavy)
+              : light_kernel<NE, 1, false>(pass, heavy);
 }
 template <int NE> void *heavy_kernel(int pass) {
   switch (pass) {
@@ -299,12 +320,10 @@ static int launch_pass(const Member *mem, int nmem, const unsigned *prefix,
     }
     nvb <<= shift;
     block = HTPB;
-  } else if (items == 2) {
-    fn = ne == 8 ? light_kernel<8, 2>(pass, heavy)
-                 : light_kernel<10, 2>(pass, heavy);
   } else {
-    fn = ne == 8 ? light_kernel<8, 1>(pass, heavy)
-                 : light_kernel<10, 1>(pass, heavy);
+    const bool full = nvb * unsigned(block) > LIGHT_WAVE;
+    fn = ne == 8 ? light_kernel<8>(pass, heavy, items, full)
+                 : light_kernel<10>(pass, heavy, items, full);
   }
   void *args[] = {&mem, &nmem, &prefix, &stage, &shift, &items};
   cudaError_t err = cudaLaunchKernel(fn, dim3(nvb), dim3(block), args, 0, st);

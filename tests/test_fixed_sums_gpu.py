@@ -74,3 +74,103 @@ def test_not_finite(bad, field):
         fine = np.isfinite(w)
         np.testing.assert_array_equal(np.isfinite(g), fine)
         assert rel_diff(np.where(fine, g, 0), np.where(fine, w, 0)) <= TOL
+
+
+# 3 nx ny K edge-levels on either side of the sizes at which the joint small
+# launches end (2^16) and the PV, vertex and divergence sums begin (2^17)
+@pytest.mark.parametrize("nx,ny,K", [(26, 28, 30), (26, 28, 31), (40, 34, 32),
+                                     (40, 34, 33), (43, 64, 16), (210, 210, 1),
+                                     (150, 146, 2)])
+@pytest.mark.parametrize("T", [0, 2, 5])
+def test_size_rule_edges(nx, ny, K, T):
+    got, want = tendency(ALL if T else dict(ALL, eddy_diff4=0.0), K, T,
+                         nx=nx, ny=ny)
+    for g, w in zip(got, want):
+        assert rel_diff(g, w) <= TOL
+
+
+@pytest.mark.parametrize("T", [1, 5])
+def test_large_with_magnitudes_beyond_the_words(T):
+    """The velocity sums where the model has them in fixed point: zeros, tiny
+    and mixed magnitudes beside ordinary ones."""
+    def edit(h, vn, tr):
+        vn[::3] = 0.0
+        vn[1::7] *= 1e-99
+        vn[2::11] *= 1e-9
+        vn[:, 7] = 0.0
+        tr[0][::2] = 0.0
+
+    got, want = tendency(ALL, 33, T, edit, nx=40, ny=34)
+    for g, w in zip(got, want):
+        assert rel_diff(g, w) <= TOL
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("field", ["tr", "vn", "h"])
+def test_large_not_finite(bad, field):
+    def edit(h, vn, tr):
+        if field == "tr":
+            tr[0, 37, 5] = bad
+        elif field == "vn":
+            vn[101, 5] = bad
+        else:
+            h[55, 5] = bad
+
+    got, want = tendency(ALL, 33, 2, edit, nx=40, ny=34)
+    for g, w in zip(got, want):
+        fine = np.isfinite(w)
+        np.testing.assert_array_equal(np.isfinite(g), fine)
+        assert rel_diff(np.where(fine, g, 0), np.where(fine, w, 0)) <= TOL
+
+
+@pytest.mark.parametrize("shape,K,T", [((8, 6), 1, 9), ((40, 34), 33, 2),
+                                       ((40, 34), 33, 6), ((26, 28), 30, 3)])
+@pytest.mark.parametrize("size", [1, 12])
+def test_batch_shapes_are_bitwise_alike(shape, K, T, size):
+    """Members with and without words, with one and two elements a thread in
+    the word-sum passes: every launch shape gives the single step's bits."""
+    import torch
+    members, single = [], []
+    for i in range(size):
+        k, t = max(1, K - 3 * (i % 5)), max(0, T - i % 3)
+        mesh, params, model, _ = build(*shape, k, dict(ALL, T=t))
+        x = state(mesh, t, 40 + i)
+        a = og.ShallowWaterState(mesh, params)
+        a.upload(*x)
+        og.RK4Stepper(model).do_step(0.0, 1.0, a)
+        single.append(a.download())
+        members.append((mesh, params, model, x))
+    states = [og.ShallowWaterState(m[0], m[1]) for m in members]
+    b = og.Batch([m[2] for m in members], states, "rk4")
+    for cfg in (None, 0, 4, 5, b.config_count() - 1):
+        if cfg is not None:
+            b.set_config(cfg)
+        for s, m in zip(states, members):
+            s.upload(*m[3])
+        b.step(0.0, 1.0, 1)
+        torch.cuda.synchronize()
+        for s, want in zip(states, single):
+            for g, w in zip(s.download(), want):
+                np.testing.assert_array_equal(g, w)
+
+
+@pytest.mark.parametrize("del4", [True, False])
+def test_one_update_where_two_tracers_leave_the_words(del4):
+    """A tracer whose own value alone is out of range keeps its sum; the same
+    cell's other tracer, with such a neighbour, takes FP64.  Each is updated
+    once."""
+    cfg = ALL if del4 else dict(ALL, eddy_diff4=0.0)
+    mesh, params, model, omd = build(10, 8, 33, dict(cfg, T=5))
+    h, vn, tr = state(mesh, 5, 31)
+    tr[1, 37, 5] = 1e150
+    tr[2, 38, 5] = 1e150  # the east neighbour of 37
+    S = og.ShallowWaterState(mesh, params)
+    S.upload(h, vn, tr)
+    og.LSRKStepper(model, 1).do_step(0.0, 1.0, S)
+    want = omd.step(h.copy(), vn.copy(), tr.copy(), 0.0, 1.0, 1, kind="lsrk",
+                    nstages=1)
+    got = S.download()
+    for g, w in zip(got[:2], want[:2]):
+        assert rel_diff(g, w) <= TOL
+    for g, w in zip(got[2], want[2]):
+        assert rel_diff(g, w) <= TOL
