@@ -20,19 +20,48 @@ constexpr int HTPB = 64;
 constexpr int HEAVY_AUX2_BLOCKS = 20, HEAVY_EDGE_BLOCKS = 12,
               HEAVY_CELL_BLOCKS = 10;
 
+// a + b and a b as multiply-adds with every operand in a register, which issue at
+// 1.90 per SM per clock: 1.60 with an operand from the constant bank or a
+// uniform register (kernel parameters, literals), and as additions and
+// products by themselves.  a 1 + b and a b + (-0) are the sum and the product
+// to the last bit; 1 and -0 come from memory.  For the passes that are FP64
+// throughout, up to half of whose instructions are sums and products: k_edge1
+// 228 -> 215 us at 256x256x64 and 20.4 -> 18.5 at 64x64x64, the RK4 step of
+// 200x230 cells with one level 105 -> 98, the tangent-linear step of 96x80x32
+// 795 -> 758.  In the passes with fixed-point sums the registers cost more
+// (k_edge_final 499 -> 514 us).
+static __device__ double2 fp64_units = {1.0, -0.0};
+__device__ __forceinline__ double fma_reg(double a, double b, double c) {
+  double r;
+  asm("fma.rn.f64 %0, %1, %2, %3;" : "=d"(r) : "d"(a), "d"(b), "d"(c));
+  return r;
+}
+__device__ __forceinline__ double mul_reg(double a, double b) {
+  return fma_reg(a, b, __ldg(&fp64_units).y);
+}
+__device__ __forceinline__ double add_reg(double a, double b) {
+  return fma_reg(a, __ldg(&fp64_units).x, b);
+}
 // Forward-mode dual number (value, tangent): the pass functions instantiated
 // with it are the exact tangent-linear model of the double instantiation
-// (the value part runs the identical operation sequence).
+// (the value part computes each sum in FP64, where the double instantiation
+// may take it in fixed point).
 using ::fma; // keep the double overload visible beside the Dual ones
-__device__ __forceinline__ Dual operator+(Dual a, Dual b) { return {a.v + b.v, a.d + b.d}; }
-__device__ __forceinline__ Dual operator+(Dual a, double b) { return {a.v + b, a.d}; }
-__device__ __forceinline__ Dual operator-(Dual a, Dual b) { return {a.v - b.v, a.d - b.d}; }
+__device__ __forceinline__ Dual operator+(Dual a, Dual b) {
+  return {add_reg(a.v, b.v), add_reg(a.d, b.d)};
+}
+__device__ __forceinline__ Dual operator+(Dual a, double b) { return {add_reg(a.v, b), a.d}; }
+__device__ __forceinline__ Dual operator-(Dual a, Dual b) {
+  return {add_reg(a.v, -b.v), add_reg(a.d, -b.d)};
+}
 __device__ __forceinline__ Dual operator-(Dual a) { return {-a.v, -a.d}; }
 __device__ __forceinline__ Dual operator*(Dual a, Dual b) {
-  return {a.v * b.v, fma(a.d, b.v, a.v * b.d)};
+  return {mul_reg(a.v, b.v), fma(a.d, b.v, mul_reg(a.v, b.d))};
 }
-__device__ __forceinline__ Dual operator*(double a, Dual b) { return {a * b.v, a * b.d}; }
-__device__ __forceinline__ Dual operator*(Dual a, double b) { return {a.v * b, a.d * b}; }
+__device__ __forceinline__ Dual operator*(double a, Dual b) {
+  return {mul_reg(a, b.v), mul_reg(a, b.d)};
+}
+__device__ __forceinline__ Dual operator*(Dual a, double b) { return b * a; }
 __device__ __forceinline__ Dual &operator+=(Dual &a, Dual b) { a = a + b; return a; }
 __device__ __forceinline__ Dual fma(double a, Dual b, Dual c) {
   return {::fma(a, b.v, c.v), ::fma(a, b.d, c.d)};
@@ -52,6 +81,11 @@ __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(
 __device__ __forceinline__ Dual mul_rn(double a, Dual b) { return a * b; }
 __device__ __forceinline__ Dual add_rn(Dual a, Dual b) { return a + b; }
 
+template <class A, class B>
+__device__ __forceinline__ Dual mul_reg(A a, B b) { return a * b; }
+template <class B>
+__device__ __forceinline__ Dual add_reg(Dual a, B b) { return a + b; }
+
 // 1/x: hardware estimate r refined by one third-order step: with the residual
 // e = 1 - x r, 1/x = r / (1 - e) = r (1 + e + e^2 + ...), so r + r (e + e^2)
 // has the relative error e^3 (the estimate's cubed) before its one rounding.
@@ -64,7 +98,7 @@ __device__ __forceinline__ Dual add_rn(Dual a, Dual b) { return a + b; }
 __device__ __forceinline__ double rcp_nr(double x) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x, r, 1.0);
+  const double e = fma(-x, r, __ldg(&fp64_units).x);
   return fma(r, fma(e, e, e), r);
 }
 __device__ __forceinline__ Dual rcp_nr(Dual x) {
@@ -241,7 +275,7 @@ __device__ __forceinline__ T entity_sum(const ModelView &p, const FxSlot *tab,
       return t;
     }
   }
-  T t = __ldg(coef + N * c) * x[size_t(__ldg(idx + N * c)) * K + k];
+  T t = mul_reg(__ldg(coef + N * c), x[size_t(__ldg(idx + N * c)) * K + k]);
 #pragma unroll
   for (int j = 1; j < N; ++j)
     t = fma(__ldg(coef + N * c + j), x[size_t(__ldg(idx + N * c + j)) * K + k],
@@ -259,7 +293,7 @@ pt_vertex(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
   const T hv = entity_sum<3, RAW, RAW_VERTEX>(p, m.kvx, m.kvh, m.cv, v, h, K, k);
   const T z = entity_sum<3, RAW, RAW_VERTEX>(p, m.cvx, m.cvr, m.ev, v, vn, K, k);
   const T r = rcp_nr(hv);
-  a.q[i] = (z + __ldg(p.f_vertex + v)) * r;
+  a.q[i] = mul_reg(add_reg(z, __ldg(p.f_vertex + v)), r);
   if (a.rhv)
     a.rhv[i] = r;
   if (p.vel_del2 | p.vel_del4)
@@ -285,7 +319,7 @@ pt_cell1(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
       a.rh[i] = r;
     for (int l = 0; l < p.ntracers; ++l) {
       const size_t t = size_t(l) * CK + i;
-      const T n = tr[t] * r;
+      const T n = mul_reg(tr[t], r);
       a.ntr[t] = n;
       if constexpr (std::is_same<T, double>::value)
         if (a.nx)
@@ -302,10 +336,10 @@ __device__ __forceinline__ void store_pv(const AuxViewT<T> &a, unsigned i, T F,
   if constexpr (std::is_same<T, double>::value)
     if (a.FGx) {
       reinterpret_cast<ulonglong2 *>(a.FGx)[i] =
-          make_ulonglong2(fx_word(F), fx_word(F * Q));
+          make_ulonglong2(fx_word(F), fx_word(mul_reg(F, Q)));
       return;
     }
-  a.G[i] = F * Q;
+  a.G[i] = mul_reg(F, Q);
 }
 
 // Edge pass 1: mean thickness, thickness flux F = mean_h vn, vn^2, edge PV
@@ -317,25 +351,26 @@ pt_edge1(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
   const int K = m.nlayers;
   const int e = int(i / unsigned(K)), k = int(i - unsigned(e) * unsigned(K));
   const int c0 = __ldg(m.ce + 2 * e), c1 = __ldg(m.ce + 2 * e + 1);
-  const T mh = half_of(h[size_t(c0) * K + k] + h[size_t(c1) * K + k]);
+  const T mh = half_of(add_reg(h[size_t(c0) * K + k], h[size_t(c1) * K + k]));
   const T u = vn[i];
-  const T F = mh * u;
+  const T F = mul_reg(mh, u);
   a.F[i] = F;
   if (a.mh) // kept by every nonlinear model and in the adjoint's tape
     a.mh[i] = mh;
   if (p.do_vn) {
     const int v0 = __ldg(m.ve + 2 * e), v1 = __ldg(m.ve + 2 * e + 1);
-    const T Q = a.q[size_t(v0) * K + k] + a.q[size_t(v1) * K + k];
+    const T Q = add_reg(a.q[size_t(v0) * K + k], a.q[size_t(v1) * K + k]);
     a.Q[i] = Q;
     store_pv(a, i, F, Q);
-    a.u2[i] = u * u;
+    a.u2[i] = mul_reg(u, u);
     if (p.vel_del2 | p.vel_del4) {
-      const T dd = a.div[size_t(c1) * K + k] - a.div[size_t(c0) * K + k];
-      const T dz = a.zeta[size_t(v1) * K + k] - a.zeta[size_t(v0) * K + k];
+      const T dd = add_reg(a.div[size_t(c1) * K + k], -a.div[size_t(c0) * K + k]);
+      const T dz =
+          add_reg(a.zeta[size_t(v1) * K + k], -a.zeta[size_t(v0) * K + k]);
       const double idc = __ldg(m.inv_dc + e);
-      a.d2u[i] = fma(dd, idc, -(dz * __ldg(m.inv_dv + e)));
+      a.d2u[i] = fma(dd, idc, -mul_reg(dz, __ldg(m.inv_dv + e)));
       if (p.vel_del4 && m.dv4_differs)
-        a.d2u4[i] = fma(dd, idc, -(dz * __ldg(m.inv_dv4 + e)));
+        a.d2u4[i] = fma(dd, idc, -mul_reg(dz, __ldg(m.inv_dv4 + e)));
     }
   }
 }
@@ -598,7 +633,7 @@ __device__ __noinline__ T masked_dissipation(const MeshView &m,
     const int v0 = __ldg(m.ve + 2 * e), v1 = __ldg(m.ve + 2 * e + 1);
     const T dd = a.d4[size_t(c1) * K + k] - a.d4[size_t(c0) * K + k];
     const T dz = a.z4[size_t(v1) * K + k] - a.z4[size_t(v0) * K + k];
-    const T l = fma(dd, idc, -(dz * __ldg(m.inv_dv + e)));
+    const T l = fma(dd, idc, -mul_reg(dz, __ldg(m.inv_dv + e)));
     t = fma(__ldg(p.c4e + e) * mk, l, t);
   }
   (void)s;
@@ -651,19 +686,19 @@ template <class T, bool LOAD> struct EdgeIn {
     return size_t(x) * m.nlayers + k;
   }
   __device__ __forceinline__ T dke() const {
-    return LOAD ? ke1 - ke0 : a.ke[at(c1)] - a.ke[at(c0)];
+    return LOAD ? ke1 - ke0 : add_reg(a.ke[at(c1)], -a.ke[at(c0)]);
   }
   __device__ __forceinline__ T dh() const {
-    return LOAD ? h1 - h0 : h[at(c1)] - h[at(c0)];
+    return LOAD ? h1 - h0 : add_reg(h[at(c1)], -h[at(c0)]);
   }
   __device__ __forceinline__ T d2u() const { return LOAD ? d2u_ : a.d2u[i]; }
   __device__ __forceinline__ T dd() const {
-    return LOAD ? d1 - d0 : a.d4[at(c1)] - a.d4[at(c0)];
+    return LOAD ? d1 - d0 : add_reg(a.d4[at(c1)], -a.d4[at(c0)]);
   }
   __device__ __forceinline__ T dz() const {
     return LOAD ? z1 - z0
-                : a.z4[at(__ldg(m.ve + 2 * e + 1))] -
-                      a.z4[at(__ldg(m.ve + 2 * e))];
+                : add_reg(a.z4[at(__ldg(m.ve + 2 * e + 1))],
+                          -a.z4[at(__ldg(m.ve + 2 * e))]);
   }
   __device__ __forceinline__ double gidc() const {
     return LOAD ? gidc_ : __ldg(p.gidc + e);
@@ -754,7 +789,7 @@ edge_final_fixed(const MeshView &m, const ModelView &p, const AuxView &a,
     if (!EARLY || !flag) {
       S1 = fx_sum(w, x, start, flag);
       const double S2 = fx_sum(w, y, start, flag);
-      t = __dadd_rn(fma(Q, S1, S2), t);
+      t = add_rn(fma(Q, S1, S2), t);
     }
   }
   if (flag) {
@@ -788,8 +823,8 @@ pt_edge_final(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
     {
       const int je = __ldg(m.eoe + NE * e);
       const double w = __ldg(m.woe + NE * e);
-      S1 = w * a.F[size_t(je) * K + k];
-      S2 = w * a.G[size_t(je) * K + k];
+      S1 = mul_reg(w, a.F[size_t(je) * K + k]);
+      S2 = mul_reg(w, a.G[size_t(je) * K + k]);
     }
 #pragma unroll
     for (int j = 1; j < NE; ++j) {
@@ -981,6 +1016,19 @@ pt_cell_final(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
+  // (the same bits either way; see mul_reg for where which is faster)
+  auto mul = [](double x, T y) {
+    if constexpr (FX)
+      return mul_rn(x, y);
+    else
+      return mul_reg(x, y);
+  };
+  auto add = [](T x, T y) {
+    if constexpr (FX)
+      return add_rn(x, y);
+    else
+      return add_reg(x, y);
+  };
   EpiIn<T> hin;
   if (p.do_h)
     hin = epilogue_in(s.ep, s.fh, i);
@@ -995,11 +1043,11 @@ pt_cell_final(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
   if (!p.off_hadv || !p.off_tr_hadv) {
 #pragma unroll
     for (int j = 0; j < MAXE; ++j)
-      w[j] = mul_rn(__ldg(m.ccdh + 6 * c + j), a.F[size_t(ej[j]) * K + k]);
-    Sa = add_rn(w[0], w[1]);
+      w[j] = mul(__ldg(m.ccdh + 6 * c + j), a.F[size_t(ej[j]) * K + k]);
+    Sa = add(w[0], w[1]);
 #pragma unroll
     for (int j = 2; j < MAXE; ++j)
-      Sa = add_rn(Sa, w[j]);
+      Sa = add(Sa, w[j]);
   }
   if (p.do_h) // -sum_j ccd_j F_j, or nothing with thickness advection off
     epilogue(s.ep, s.fh, i, p.off_hadv ? T{} : twice(Sa), hin);
@@ -1020,14 +1068,14 @@ pt_cell_final(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
     T b[MAXE], Sb;
 #pragma unroll
     for (int j = 0; j < MAXE; ++j) {
-      b[j] = mul_rn(__ldg(p.kd2 + 6 * c + j), a.mh[size_t(ej[j]) * K + k]);
-      w[j] = add_rn(w[j], b[j]);
+      b[j] = mul(__ldg(p.kd2 + 6 * c + j), a.mh[size_t(ej[j]) * K + k]);
+      w[j] = add(w[j], b[j]);
     }
-    Sb = add_rn(b[0], b[1]);
+    Sb = add(b[0], b[1]);
 #pragma unroll
     for (int j = 2; j < MAXE; ++j)
-      Sb = add_rn(Sb, b[j]);
-    wc = add_rn(Sa, -Sb);
+      Sb = add(Sb, b[j]);
+    wc = add(Sa, -Sb);
   }
   // del4 centre weight: -sum r4, plus eddy_diff2 s when del2 is folded in
   const double rc = !del4 ? 0.0 : fold ? __ldg(p.r4f + c)
@@ -1050,7 +1098,7 @@ pt_cell_final(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
   for (; PAIRS && l + 1 < p.ntracers; l += 2) {
     const size_t b0 = size_t(l) * CK, b1 = b0 + CK;
     const T *n0 = a.ntr + b0, *n1 = a.ntr + b1;
-    T acc0 = wc * n0[i], acc1 = wc * n1[i];
+    T acc0 = mul_reg(wc, n0[i]), acc1 = mul_reg(wc, n1[i]);
 #pragma unroll
     for (int j = 0; j < MAXE; ++j) {
       acc0 = fma(w[j], n0[off[j]], acc0);
