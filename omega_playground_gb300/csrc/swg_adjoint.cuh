@@ -69,7 +69,7 @@ struct AdjIO {
 };
 
 // The adds here and in the passes that take a product (x is often one) are
-// written as __dadd_rn: the compiler may not fuse them into a multiply-add,
+// written as add_reg or __dadd_rn: the compiler may not fuse them into a multiply-add,
 // which it could otherwise do differently in the single-instance and the
 // batched kernels that inline the same pass, and the two must agree bit for
 // bit.
@@ -81,7 +81,7 @@ __device__ __forceinline__ void emit(const AdjIO &io, double *out,
     out[i] = x;
   double a = 0;
   if (acc) {
-    a = __dadd_rn(acc_in[i], x);
+    a = add_reg(acc_in[i], x);
     acc[i] = a;
   }
   if (nmu) {
@@ -97,7 +97,7 @@ __device__ __forceinline__ void emit(const AdjIO &io, double *out,
       c = io.gamma;
       y = mu[i];
     }
-    nmu[i] = fma(io.alpha, u, c * y);
+    nmu[i] = fma(io.alpha, u, mul_reg(c, y));
   }
 }
 
@@ -128,7 +128,7 @@ pa_vel(const MeshView &m, const ModelView &p, const AuxView &a,
   if (i >= VK + CK) {
     i -= VK + CK;
     if (i < unsigned(m.nedges) * K && !p.off_pv)
-      w.Qmu[i] = a.Q[i] * io.mvn[i];
+      w.Qmu[i] = mul_reg(a.Q[i], io.mvn[i]);
     return;
   }
   // the del4 term is masked per edge and level (mask * c4e): its
@@ -234,7 +234,7 @@ pa_tr1(const MeshView &m, const ModelView &p, const AuxView &a,
     double x = 0;
     if (adv) {
       const double F = a.F[size_t(e) * K + k];
-      x = __ldg(v.ccdh_nb + 6 * c + j) * F;
+      x = mul_reg(__ldg(v.ccdh_nb + 6 * c + j), F);
       wc = fma(__ldg(m.ccdh + 6 * c + j), F, wc);
     }
     if (D2) {
@@ -246,12 +246,12 @@ pa_tr1(const MeshView &m, const ModelView &p, const AuxView &a,
   }
   for (int l = 0; l < p.ntracers; ++l) {
     const double *mu = io.mtr + size_t(l) * CK;
-    double acc = wc * mu[i];
+    double acc = mul_reg(wc, mu[i]);
     for (int j = 0; j < MAXE; ++j)
       acc = fma(wnb[j], mu[size_t(nb[j]) * K + k], acc);
     w.ln[size_t(l) * CK + i] = acc;
     if (D4) {
-      double L = -__ldg(p.r4sum + c) * mu[i];
+      double L = mul_reg(-__ldg(p.r4sum + c), mu[i]);
       for (int j = 0; j < MAXE; ++j)
         L = fma(__ldg(v.r4_nb + 6 * c + j), mu[size_t(nb[j]) * K + k], L);
       w.lL[size_t(l) * CK + i] = L;
@@ -277,7 +277,7 @@ pa_tr2(const MeshView &m, const ModelView &p, const AuxView &a,
       const int e = __ldg(m.ec + 6 * c + j);
       const double mh = mean_h(m, a, io.h, e, k);
       nb[j] = __ldg(m.nbc + 6 * c + j);
-      mnb[j] = __ldg(v.ckq_nb + 6 * c + j) * mh;
+      mnb[j] = mul_reg(__ldg(v.ckq_nb + 6 * c + j), mh);
       M = fma(__ldg(m.ckq + 6 * c + j), mh, M);
     }
   // 1/h: the forward's own reciprocal (taped, or recomputed)
@@ -293,10 +293,10 @@ pa_tr2(const MeshView &m, const ModelView &p, const AuxView &a,
         ln = fma(mnb[j], lL[size_t(nb[j]) * K + k], ln);
     }
     emit(io, io.ltr, io.acc_in_tr, io.acc_tr, io.nmu_tr, io.lam_tr, io.mtr, t,
-         ln * r);
+         mul_reg(ln, r));
     hsum = fma(ln, a.ntr[t], hsum);
   }
-  w.lhtr[i] = -(r * hsum);
+  w.lhtr[i] = -mul_reg(r, hsum);
 }
 
 // mu times the edge mask of element i
@@ -335,7 +335,7 @@ pa_edge(const MeshView &m, const ModelView &p, const AuxView &a,
       }
       // (S1 may be lQ itself, see adj_tendency)
       const double S1 = a.S1 ? a.S1[i] : s1_of<NE>(m, a, e, k);
-      w.lQ[i] = fma(S1, mu, F * lG);
+      w.lQ[i] = fma(S1, mu, mul_reg(F, lG));
       lF = fma(a.Q[i], lG, lFq);
     } else {
       w.lQ[i] = 0.0;
@@ -343,8 +343,8 @@ pa_edge(const MeshView &m, const ModelView &p, const AuxView &a,
     // kinetic energy from vn^2 (the factor 2 of d(vn^2) is in cke2_e2)
     if (!p.off_ke) {
       const double lu2 = fma(__ldg(v.cke2_e2 + 2 * e), w.lke[i0],
-                             __ldg(v.cke2_e2 + 2 * e + 1) * w.lke[i1]);
-      w.lvnp[i] = u * lu2; // mean-h term added below
+                             mul_reg(__ldg(v.cke2_e2 + 2 * e + 1), w.lke[i1]));
+      w.lvnp[i] = mul_reg(u, lu2); // mean-h term added below
     } else {
       w.lvnp[i] = 0.0;
     }
@@ -352,7 +352,7 @@ pa_edge(const MeshView &m, const ModelView &p, const AuxView &a,
       // the dissipation terms are masked per edge and level (no multiply
       // without a mask)
       const double mum = m.mask ? masked(mu, m.mask, i) : mu;
-      const double d = p.vel_del2 ? __ldg(p.c2e + e) * mum : 0.0;
+      const double d = p.vel_del2 ? mul_reg(__ldg(p.c2e + e), mum) : 0.0;
       if (p.vel_del2 && w.gc2e) // parameter gradient of the del2 coefficient
         w.gc2e[i] = fma(mum, a.d2u[i], w.gc2e[i]);
       if (p.vel_del4) {
@@ -389,15 +389,16 @@ pa_edge(const MeshView &m, const ModelView &p, const AuxView &a,
     const double n0 = a.ntr[b + i0], n1 = a.ntr[b + i1];
     const double m0 = io.mtr[b + i0], m1 = io.mtr[b + i1];
     if (adv)
-      lF = fma(n0 + n1, fma(g0, m0, g1 * m1), lF);
+      lF = fma(add_reg(n0, n1), fma(g0, m0, mul_reg(g1, m1)), lF);
     if (TRD) {
-      const double dn = n1 - n0;
+      const double dn = add_reg(n1, -n0);
       if (p.tr_del2)
         lmh = fma(dn, fma(__ldg(v.kd2_e2 + 2 * e), m0,
-                          -(__ldg(v.kd2_e2 + 2 * e + 1) * m1)), lmh);
+                          -mul_reg(__ldg(v.kd2_e2 + 2 * e + 1), m1)), lmh);
       if (p.tr_del4)
         lmh = fma(dn, fma(__ldg(v.ckq_e2 + 2 * e), w.lL[b + i0],
-                          -(__ldg(v.ckq_e2 + 2 * e + 1) * w.lL[b + i1])), lmh);
+                          -mul_reg(__ldg(v.ckq_e2 + 2 * e + 1), w.lL[b + i1])),
+                  lmh);
     }
   }
   const double mh = mean_h(m, a, io.h, e, k);
@@ -462,11 +463,12 @@ pa_vertex(const MeshView &m, const ModelView &p, const AuxView &a,
   const int vx = int(i / unsigned(K)), k = int(i - unsigned(vx) * K);
   const int e0 = __ldg(m.ev + 3 * vx), e1 = __ldg(m.ev + 3 * vx + 1),
             e2 = __ldg(m.ev + 3 * vx + 2);
-  const double lq = w.lQ[size_t(e0) * K + k] + w.lQ[size_t(e1) * K + k] +
-                    w.lQ[size_t(e2) * K + k];
+  const double lq = add_reg(
+      add_reg(w.lQ[size_t(e0) * K + k], w.lQ[size_t(e1) * K + k]),
+      w.lQ[size_t(e2) * K + k]);
   double lz = 0;
   if (p.vel_del2 | p.vel_del4) {
-    lz = __ldg(v.zetaadj + 3 * vx) * w.ld2u[size_t(e0) * K + k];
+    lz = mul_reg(__ldg(v.zetaadj + 3 * vx), w.ld2u[size_t(e0) * K + k]);
     lz = fma(__ldg(v.zetaadj + 3 * vx + 1), w.ld2u[size_t(e1) * K + k], lz);
     lz = fma(__ldg(v.zetaadj + 3 * vx + 2), w.ld2u[size_t(e2) * K + k], lz);
     if (w.ld2u4) // the del4 chain's part, with 1/max(dv, dc/4)
@@ -475,7 +477,7 @@ pa_vertex(const MeshView &m, const ModelView &p, const AuxView &a,
   // 1/h_vertex: the forward's value (taped, or recomputed)
   const double r = a.rhv ? a.rhv[i] : vertex_rcp(m, io.h, vx, k);
   w.lzeta[i] = fma(r, lq, lz);
-  w.lhv[i] = -(a.q[i] * r * lq);
+  w.lhv[i] = -mul_reg(mul_reg(a.q[i], r), lq);
 }
 
 // --- pass 6: cells: thickness adjoint.
@@ -497,7 +499,7 @@ pa_cell(const MeshView &m, const ModelView &p, const AuxView &a,
   if (p.do_vn && !p.off_ssh)
     lh = fma(p.grav, w.lke[i], lh); // SSH gradient: g times the KE term
   if (p.ntracers > 0)
-    lh = __dadd_rn(lh, w.lhtr[i]);
+    lh = add_reg(lh, w.lhtr[i]);
   emit(io, io.lh, io.acc_in_h, io.acc_h, io.nmu_h, io.lam_h, io.mh_, i, lh);
 }
 
