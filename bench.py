@@ -39,12 +39,13 @@ METRIC = ("cell·level·stage updates/s FP64 (% HBM roofline); "
 UNIT = "cell·level·stage updates/s"
 PEAKS_FILE = os.path.join(ROOT, "MEASURED_PEAKS.json")
 FALLBACK_HBM_GBS = 6800.0
-# FP64 thread instructions (DFMA + DADD + DMUL) per cell-level of
-# k_cell_final on the LSRK5 512x512x64x8 workload's physics, counted by ncu
-# (smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on.sum over the
-# launch's cell-levels); it is a property of the compiled kernel and the
-# enabled terms, not of the mesh size
-K_CELL_FINAL_FP64 = 142
+# FP64-pipe thread instructions per cell-level of the cell final pass
+# (k_cell_tracers) on the LSRK5 512x512x64x8 workload's physics, counted by ncu
+# (32 smsp__inst_executed_pipe_fp64.sum over the launch's cell-levels: DFMA +
+# DADD + DMUL 45, and 9 conversions of fixed-point sums); it is a property of
+# the compiled kernel and the enabled terms, not of the mesh size.  The pass's
+# 12-term sums are integer instructions: this fraction is the FP64 pipe's share
+K_CELL_FINAL_FP64 = 54
 
 
 def parse():
@@ -426,10 +427,10 @@ def run_ours(args, wl):
     achieved = dom_bytes / (dom_ms / 1e3) / 1e9
     stage_bytes = wl.alg_bytes_per_stage()
     # DRAM bytes per cell-level of the dominant kernel from one ncu capture
-    # (dram__bytes_read.sum + dram__bytes_write.sum of k_cell_final on the
-    # 256x256x64x8 case: 1.932 GB for 4,194,304 cell-levels), scaled to
+    # (dram__bytes_read.sum + dram__bytes_write.sum of k_cell_tracers on the
+    # 256x256x64x8 case: 2.376 GB for 4,194,304 cell-levels), scaled to
     # this launch by its cell-level count; traffic grows in proportion.
-    ncu_bytes_per_unit = {"k_cell_final": 1.932e9 / 4194304}
+    ncu_bytes_per_unit = {"k_cell_final": 2.376e9 / 4194304}
     traffic = (ncu_bytes_per_unit[dom] * CK
                if dom in ncu_bytes_per_unit and wl.ntracers == 8 else None)
     roofline = {"bound": "hbm", "kernel": dom, "achieved": achieved,
@@ -443,8 +444,8 @@ def run_ours(args, wl):
     # FP64 issue roof, measured here: DFMA / DADD / DMUL issue rates of this
     # GPU (swg_fp64_issue_rate: every SM filled, 4 independent chains per
     # thread, CUDA events) with the SM clock sampled while they run.  The
-    # instructions per cell-level of k_cell_final come from ncu on the
-    # 256x256x64x8 case (DFMA 132 + DMUL 15 + DADD 8 = 155 with 8 tracers).
+    # FP64-pipe instructions per cell-level of the cell final pass come from
+    # ncu on the 256x256x64x8 case.
     fp64 = None
     if dom == "k_cell_final" and wl.ntracers == 8:
         sms = torch.cuda.get_device_properties(local).multi_processor_count

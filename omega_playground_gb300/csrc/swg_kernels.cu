@@ -11,8 +11,13 @@
 //    (loaded as warp-broadcasts) and zero TRiSK weights are dropped;
 //  - tracer terms are rewritten as weighted sums over neighbour values whose
 //    weights are shared by all tracers of a cell;
-//  - reciprocals use Newton-Raphson from the hardware approximation (5 FP64
-//    slots instead of about 9 for IEEE division);
+//  - the wide sums (PV flux, tracers, tracer Laplacians; in large models also
+//    the vertex and divergence sums) run on the integer pipes in fixed point
+//    (swg_fixed.cuh), which idle beside FP64;
+//  - sums and products by themselves are multiply-adds with all operands in
+//    registers, which issue faster (mul_reg, swg_device.cuh);
+//  - reciprocals are one third-order step from the hardware approximation (3
+//    FP64 instructions instead of about 9 for IEEE division);
 //  - the RK stage update is fused into the last two kernels.
 // One thread handles one (entity, level); k is the fastest index, so a warp
 // reads 32 consecutive levels (256 contiguous bytes) of one entity.
@@ -27,7 +32,7 @@
 //   k_edge_final pv_flux_edge.hpp:149-177, ke_grad_edge.hpp:223-237,
 //               ssh_grad_edge.hpp:281-294, vel_diff_edge.hpp:61-86,
 //               vel_hyperdiff_edge.hpp:309-334, rk4.cpp:94-138, lsrk.cpp:47-86
-//   k_cell_final thickness_hadv_cell.hpp:59-83, tracer_hadv_cell.hpp:60-90,
+//   k_cell_final (k_cell_tracers with fixed-point sums) thickness_hadv_cell.hpp:59-83, tracer_hadv_cell.hpp:60-90,
 //               tracer_diff_cell.hpp:162-193, tracer_hyperdiff_cell.hpp:338-368
 #include "swg_device.cuh"
 
