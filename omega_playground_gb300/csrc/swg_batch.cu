@@ -163,14 +163,21 @@ __device__ __forceinline__ int member_of(const unsigned *pre, int nmem,
 // Laplacian in FP64.  The vertex and the first edge pass are held to 32
 // registers, 64 warps per SM (12 members, 2 elements a thread: 86 us with 40
 // and 80 with 32, 155 us with 38 and 141 with 32).
-// FULL: not where 48 warps per SM hold all of the pass's elements: there a
-// thread's loads in flight count (gradients of 3 members 12x8x33, 3 steps:
-// 932 us with it, 901 without).
-template <int PASS, bool FULL> constexpr int light_blocks() {
-  return FULL && (PASS == P_VERTEX || PASS == P_EDGE1) ? 4 : 0;
+// That is SIZE 2, more threads than 48 warps on each SM hold; with fewer a
+// thread's loads in flight count, and there is no bound (SIZE 1: gradients of
+// 3 members 12x8x33, 3 steps, 932 us with the bound and 901 without).  SIZE 0:
+// one block of 256 threads on each SM holds the pass, and the bound of one
+// block lets the compiler take 45-52 registers (4 members to 17x16x40: 939 us
+// without, 909 with; 4 members to 48x48x32, of more threads, 7.03 ms without
+// and 7.15 with).
+template <int PASS, int SIZE> constexpr int light_blocks() {
+  return PASS != P_VERTEX && PASS != P_EDGE1 ? 0
+         : SIZE == 2                         ? 4
+         : SIZE == 1                         ? 0
+                                             : 1;
 }
-template <int NE, int ITEMS, int PASS, int RAW, bool FULL>
-__global__ void __launch_bounds__(512, light_blocks<PASS, FULL>())
+template <int NE, int ITEMS, int PASS, int RAW, int SIZE>
+__global__ void __launch_bounds__(512, light_blocks<PASS, SIZE>())
     k_batch_pass(const Member *__restrict__ mem, int nmem,
                  const unsigned *__restrict__ prefix, int stage) {
   const unsigned vbsize = blockDim.x * ITEMS;
@@ -205,6 +212,8 @@ __global__ void __launch_bounds__(512, light_blocks<PASS, FULL>())
 constexpr unsigned HEAVY_WAVE = 1520;
 // threads of 48 warps on each SM
 constexpr unsigned LIGHT_WAVE = 152 * 1536;
+// threads of one block of 256 on each SM
+constexpr unsigned LIGHT_BLOCK = 152 * 256;
 template <int PASS> constexpr int heavy_blocks() {
   return PASS == P_AUX2 ? HEAVY_AUX2_BLOCKS
          : PASS == P_CELL_FINAL ? HEAVY_CELL_BLOCKS
@@ -235,47 +244,46 @@ __global__ void __launch_bounds__(HTPB, heavy_blocks<PASS>())
   }
 }
 
-template <int NE, int ITEMS, int RAW, bool FULL>
+template <int NE, int ITEMS, int RAW, int SIZE>
 void *light_kernel(int pass) {
   switch (pass) {
   case P_VERTEX:
     return reinterpret_cast<void *>(
-        &k_batch_pass<NE, ITEMS, P_VERTEX, RAW, FULL>);
+        &k_batch_pass<NE, ITEMS, P_VERTEX, RAW, SIZE>);
   case P_CELL1:
     return reinterpret_cast<void *>(
-        &k_batch_pass<NE, ITEMS, P_CELL1, RAW, true>);
+        &k_batch_pass<NE, ITEMS, P_CELL1, RAW, 2>);
   case P_EDGE1:
     return reinterpret_cast<void *>(
-        &k_batch_pass<NE, ITEMS, P_EDGE1, 0, FULL>);
+        &k_batch_pass<NE, ITEMS, P_EDGE1, 0, SIZE>);
   case P_AUX2:
     return reinterpret_cast<void *>(
-        &k_batch_pass<NE, ITEMS, P_AUX2, RAW == 1, true>);
+        &k_batch_pass<NE, ITEMS, P_AUX2, RAW == 1, 2>);
   case P_EDGE_FINAL:
     return reinterpret_cast<void *>(
-        &k_batch_pass<NE, ITEMS, P_EDGE_FINAL, 0, true>);
+        &k_batch_pass<NE, ITEMS, P_EDGE_FINAL, 0, 2>);
   default:
     return reinterpret_cast<void *>(
-        &k_batch_pass<NE, ITEMS, P_CELL_FINAL, 0, true>);
+        &k_batch_pass<NE, ITEMS, P_CELL_FINAL, 0, 2>);
   }
 }
-template <int NE, int ITEMS, bool FULL>
+template <int NE, int ITEMS, int SIZE>
 void *light_kernel(int pass, unsigned heavy) {
   if (pass == P_AUX2)
-    return heavy & HEAVY_LAP || !FULL ? light_kernel<NE, ITEMS, 0, FULL>(pass)
-                                      : light_kernel<NE, ITEMS, 1, FULL>(pass);
+    return heavy & HEAVY_LAP || SIZE < 2
+               ? light_kernel<NE, ITEMS, 0, SIZE>(pass)
+               : light_kernel<NE, ITEMS, 1, SIZE>(pass);
   if (!(heavy & HEAVY_RAW))
-    return light_kernel<NE, ITEMS, 0, FULL>(pass);
+    return light_kernel<NE, ITEMS, 0, SIZE>(pass);
   if (heavy & HEAVY_NO_RAW) // members of both kinds
-    return light_kernel<NE, ITEMS, -1, FULL>(pass);
-  return light_kernel<NE, ITEMS, 1, FULL>(pass);
+    return light_kernel<NE, ITEMS, -1, SIZE>(pass);
+  return light_kernel<NE, ITEMS, 1, SIZE>(pass);
 }
-template <int NE>
-void *light_kernel(int pass, unsigned heavy, int items, bool full) {
-  if (items == 2)
-    return full ? light_kernel<NE, 2, true>(pass, heavy)
-                : light_kernel<NE, 2, false>(pass, heavy);
-  return full ? light_kernel<NE, 1, true>(pass, heavy)
-              : light_kernel<NE, 1, false>(pass, heavy);
+template <int NE, int ITEMS>
+void *light_kernel(int pass, unsigned heavy, unsigned threads) {
+  return threads > LIGHT_WAVE    ? light_kernel<NE, ITEMS, 2>(pass, heavy)
+         : threads > LIGHT_BLOCK ? light_kernel<NE, ITEMS, 1>(pass, heavy)
+                                 : light_kernel<NE, ITEMS, 0>(pass, heavy);
 }
 template <int NE> void *heavy_kernel(int pass) {
   switch (pass) {
@@ -321,9 +329,13 @@ static int launch_pass(const Member *mem, int nmem, const unsigned *prefix,
     nvb <<= shift;
     block = HTPB;
   } else {
-    const bool full = nvb * unsigned(block) > LIGHT_WAVE;
-    fn = ne == 8 ? light_kernel<8>(pass, heavy, items, full)
-                 : light_kernel<10>(pass, heavy, items, full);
+    const unsigned threads = nvb * unsigned(block);
+    if (items == 2)
+      fn = ne == 8 ? light_kernel<8, 2>(pass, heavy, threads)
+                   : light_kernel<10, 2>(pass, heavy, threads);
+    else
+      fn = ne == 8 ? light_kernel<8, 1>(pass, heavy, threads)
+                   : light_kernel<10, 1>(pass, heavy, threads);
   }
   void *args[] = {&mem, &nmem, &prefix, &stage, &shift, &items};
   cudaError_t err = cudaLaunchKernel(fn, dim3(nvb), dim3(block), args, 0, st);
