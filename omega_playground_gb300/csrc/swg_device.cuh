@@ -981,8 +981,13 @@ tracer_sums(const MeshView &m, const ModelView &p, const AuxView &a,
     if (!flag)
       epilogue(s.ep, s.ftr, base + off[MAXE], acc, in);
   }
-  if (redo)
+  if (redo) {
+    // a bad weight left the first tracer's copies in flight: the thread's
+    // next element (k_batch_heavy) copies to the same slots
+    if (ASYNC)
+      asm volatile("cp.async.wait_all;" ::: "memory");
     tracers_f64(m, p, a, s, c, k, bad != 0);
+  }
 }
 
 // Cell final pass: thickness tendency and tracer tendencies (advection,

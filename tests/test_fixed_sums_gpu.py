@@ -174,3 +174,34 @@ def test_one_update_where_two_tracers_leave_the_words(del4):
         assert rel_diff(g, w) <= TOL
     for g, w in zip(got[2], want[2]):
         assert rel_diff(g, w) <= TOL
+
+
+@pytest.mark.parametrize("T,del4", [(1, True), (3, True), (3, False)])
+def test_bad_weights_beside_finite_elements_in_a_batch(T, del4):
+    """Batches large enough for two elements a thread in the word-sum passes:
+    a cell whose weights are not finite skips its sums, and the thread's next
+    element has the single step's bits all the same."""
+    import torch
+    cfg = ALL if del4 else dict(ALL, eddy_diff4=0.0)
+    members, single = [], []
+    for i in range(4):
+        mesh, params, model, _ = build(40, 34, 33, dict(cfg, T=T))
+        h, vn, tr = state(mesh, T, 60 + i)
+        vn[i::37, 3::5] = np.nan
+        vn[9::53, i] = np.inf
+        vn[20::71, 2 * i + 1] = 1e-200  # F, and so the weight, below 2^-400
+        a = og.ShallowWaterState(mesh, params)
+        a.upload(h, vn, tr)
+        og.LSRKStepper(model, 1).do_step(0.0, 1.0, a)
+        single.append(a.download())
+        assert np.isfinite(single[-1][2]).any()
+        members.append((mesh, params, model, (h, vn, tr)))
+    states = [og.ShallowWaterState(m[0], m[1]) for m in members]
+    for s, m in zip(states, members):
+        s.upload(*m[3])
+    b = og.Batch([m[2] for m in members], states, "lsrk", 1)
+    b.step(0.0, 1.0, 1)
+    torch.cuda.synchronize()
+    for s, want in zip(states, single):
+        for g, w in zip(s.download(), want):
+            np.testing.assert_array_equal(g, w)
