@@ -93,7 +93,7 @@ __global__ void k_edge_terms(MeshView m, int ne, FxSlot *out, long long *start,
   long long sum = 0;
   unsigned flag = 0;
   for (int j = 0; j < ne; ++j) {
-    const FxSlot t{m.eoe[ne * e + j], fx_weight(m.woe[ne * e + j], flag)};
+    const FxSlot t{m.eoe[ne * e + j], fx_weight<FX_TOP>(m.woe[ne * e + j], flag)};
     out[ne * e + j] = t;
     sum += t.w.hi;
   }

@@ -440,8 +440,37 @@ static __device__ __noinline__ double pv_flux_f64(const MeshView &m,
   return fma(a.Q[i], S1, S2);
 }
 
+// Whether a tracer's sum over the words n (and with del4 L) of the neighbours
+// is left to FP64: the decision of fx_sum, from the same weights.  Not an extra
+// register of the tracer loop: there a mask of the tracers costs more than
+// reading the words again here (k_cell_tracers with 8 tracers 630 -> 700 us at
+// 256x256x64).
+__device__ __forceinline__ bool
+tracer_left(const fx_t *n, const fx_t *L, bool del4, const double (&w)[MAXE],
+            const double (&r4)[MAXE], const unsigned (&off)[MAXE]) {
+  fx_t x[MAXE], y[MAXE];
+  unsigned f = 0, unused = 0;
+#pragma unroll
+  for (int j = 0; j < MAXE; ++j) {
+    x[j] = n[off[j]];
+    y[j] = del4 ? L[off[j]] : 0;
+    f |= unsigned(x[j]) | unsigned(y[j]);
+  }
+  if (f & FX_FLAG)
+    return true;
+  int P = FX_ZERO_EXP;
+#pragma unroll
+  for (int j = 0; j < MAXE; ++j) {
+    P = max(P, fx_exp(x[j], fx_weight<FX_TOP>(w[j], unused).e));
+    if (del4)
+      P = max(P, fx_exp(y[j], fx_weight<FX_TOP>(r4[j], unused).e));
+  }
+  return fx_left(P, FX_TOP, f) != 0;
+}
+
 // flux divergence, diffusion and hyperdiffusion at cell c, and the stage
-// update, of every tracer (all) or of those with a flagged word
+// update, of every tracer (all) or of those that tracer_sums left here: the
+// weights w are its own to the last bit
 static __device__ __noinline__ void tracers_f64(const MeshView &m,
                                                 const ModelView &p,
                                                 const AuxView &a,
@@ -458,12 +487,12 @@ static __device__ __noinline__ void tracers_f64(const MeshView &m,
     off[j] = unsigned(__ldg(m.nbc + 6 * c + j)) * unsigned(K) + unsigned(k);
     w[j] = r4[j] = 0;
     if (!p.off_tr_hadv) {
-      w[j] = __ldg(m.ccdh + 6 * c + j) * a.F[ie];
+      w[j] = mul_rn(__ldg(m.ccdh + 6 * c + j), a.F[ie]);
       wc += w[j];
     }
     if (p.tr_del2 && !fold) {
-      const double b = __ldg(p.kd2 + 6 * c + j) * a.mh[ie];
-      w[j] += b;
+      const double b = mul_rn(__ldg(p.kd2 + 6 * c + j), a.mh[ie]);
+      w[j] = add_rn(w[j], b);
       wc -= b;
     }
     if (p.tr_del4)
@@ -474,17 +503,9 @@ static __device__ __noinline__ void tracers_f64(const MeshView &m,
 #pragma unroll 1
   for (int l = 0; l < p.ntracers; ++l) {
     const size_t base = size_t(l) * (unsigned(m.ncells) * unsigned(K));
-    if (!all) {
-      unsigned flag = 0;
-#pragma unroll
-      for (int j = 0; j < MAXE; ++j) {
-        flag |= unsigned(a.nx[base + off[j]]);
-        if (p.tr_del4)
-          flag |= unsigned(a.lx[base + off[j]]);
-      }
-      if (!(flag & FX_FLAG))
-        continue;
-    }
+    if (!all &&
+        !tracer_left(a.nx + base, a.lx + base, p.tr_del4, w, r4, off))
+      continue;
     const double *n = a.ntr + base, *L = a.lap + base;
     double acc = 0;
 #pragma unroll
@@ -556,7 +577,7 @@ __device__ __forceinline__ void pt_aux2(const MeshView &m, const ModelView &p,
       long long start = 0;
 #pragma unroll
       for (int j = 0; j <= MAXE; ++j) {
-        W[j] = fx_weight(j < MAXE ? w[j < MAXE ? j : 0] : -M, bad);
+        W[j] = fx_weight<FX_TOP>(j < MAXE ? w[j < MAXE ? j : 0] : -M, bad);
         start += W[j].hi;
       }
       start = fx_start(start);
@@ -575,7 +596,8 @@ __device__ __forceinline__ void pt_aux2(const MeshView &m, const ModelView &p,
 #pragma unroll
           for (int j = 0; j <= MAXE; ++j)
             x[j] = n[off[j]];
-          const double L = fx_sum(W, x, start, redo);
+          const double L =
+              fx_sum<MAXE + 1, false>(W, x, start, FX_TOP, redo);
           a.lap[base + i] = L;
           a.lx[base + i] = fx_word(L);
         }
@@ -787,8 +809,8 @@ edge_final_fixed(const MeshView &m, const ModelView &p, const AuxView &a,
     if (EARLY)
       flag = unsigned(x[0]) & FX_FLAG;
     if (!EARLY || !flag) {
-      S1 = fx_sum(w, x, start, flag);
-      const double S2 = fx_sum(w, y, start, flag);
+      S1 = fx_sum<NE, true>(w, x, start, FX_TOP, flag);
+      const double S2 = fx_sum<NE, true>(w, y, start, FX_TOP, flag);
       t = add_rn(fma(Q, S1, S2), t);
     }
   }
@@ -860,7 +882,7 @@ __device__ __forceinline__ void pt_pv_sum(const MeshView &m, const AuxView &a,
       w[j] = {s4.y, s4.z, s4.w};
       x[j] = a.FGx[2 * size_t(unsigned(s4.x) * K + unsigned(k))];
     }
-    S1 = fx_sum(w, x, __ldg(m.fxe0 + e), flag);
+    S1 = fx_sum<NE, true>(w, x, __ldg(m.fxe0 + e), FX_TOP, flag);
   }
   if (flag) {
     S1 = 0;
@@ -925,7 +947,7 @@ tracer_sums(const MeshView &m, const ModelView &p, const AuxView &a,
   long long start = 0;
 #pragma unroll
   for (int j = 0; j < MAXE; ++j) {
-    W[j] = fx_weight(w[j], bad);
+    W[j] = fx_weight<FX_TOP>(w[j], bad);
     start += W[j].hi;
   }
   if (D4) {
@@ -974,7 +996,7 @@ tracer_sums(const MeshView &m, const ModelView &p, const AuxView &a,
       in = epilogue_in(s.ep, s.ftr, base + off[MAXE]);
     }
     unsigned flag = 0;
-    double acc = fma(wc, nc, fx_sum(W, x, start, flag));
+    double acc = fma(wc, nc, fx_sum<N, false>(W, x, start, FX_TOP, flag));
     if (D4)
       acc = fma(rc, Lc, acc);
     redo |= flag;

@@ -24,10 +24,15 @@
 // accumulated in 64 bits.  With M the largest |w_j x_j|: the shifts drop at
 // most 2^-59 M per term, the product lo x (low half) at most 2^-56 M per
 // term (rms below 2^-57.5, of either sign as lo is), and the final rounding
-// 2^-56 M.  A chain of FP64 multiply-adds
-// rounds by up to 2^-53 of each partial sum, so the sum is the more accurate
-// of the two for any mixture of magnitudes and signs; a sum of zero products
-// is exactly zero.
+// 2^-56 M.  A chain of FP64 multiply-adds rounds by up to 2^-53 of each
+// partial sum; a sum of zero products is exactly zero.
+//
+// A zero has no exponent: its word gives the product the exponent e_j of its
+// weight alone, which could shift smaller products out (2^-314 of that weight
+// and less).  Where the largest exponent is no more than a bound `top` of the
+// e_j and some word is not zero, the sum leaves the zeros' exponents out (LOW),
+// or it is left to FP64 with those below.  The passes take weights below 2^36
+// and the constant FX_TOP: only sums with M below 2^-278 are looked at again.
 //
 // A term that cannot be represented (a flagged word, or a weight out of
 // range) makes the caller evaluate that one sum in FP64 instead: infinities
@@ -49,6 +54,7 @@ using fx_t = unsigned long long;
 constexpr unsigned FX_FLAG = 0x80; // low-byte bit of an unrepresentable value
 constexpr int FX_ZERO_EXP = -100000; // exponent of a zero weight
 constexpr int FX_BAD_EXP = 100000;   // and of a table's out-of-range weight
+constexpr int FX_TOP = -20;          // largest exponent of a pass's weight
 constexpr int FX_SCALE = -317;       // 60 - 377: result exponent offset
 
 struct Wt {
@@ -83,8 +89,10 @@ SWG_HD long long fx_sar(long long x, unsigned s) {
 #endif
 }
 
-// The weight w; sets FX_FLAG in `flag` when it is out of range.
-SWG_HD Wt fx_weight(double w, unsigned &flag) {
+// The weight w; sets FX_FLAG in `flag` when it is out of range, or its exponent
+// above TOP.
+template <int TOP = 345> SWG_HD Wt fx_weight(double w, unsigned &flag) {
+  static_assert(TOP <= 345, "2^400");
   const fx_t b = fx_bits(w);
   const int eb = int(unsigned(b >> 52) & 0x7ff);
   const long long s = (long long)b >> 63;
@@ -94,7 +102,7 @@ SWG_HD Wt fx_weight(double w, unsigned &flag) {
   r.hi = int((W + (1LL << 27)) >> 28);
   r.lo = int(unsigned(W) << 4) >> 4;
   r.e = eb - 1078;
-  if (unsigned(eb - 623) > 800u) { // |w| outside 2^-400 .. 2^400
+  if (unsigned(eb - 623) > unsigned(TOP + 455)) { // |w| below 2^-400, or above
     if (!fx_is_zero(b))
       flag |= FX_FLAG;
     r.hi = r.lo = 0;
@@ -122,7 +130,7 @@ SWG_HD fx_t fx_word(double x) {
 // The weight w for a table: exponent FX_BAD_EXP when it is out of range.
 SWG_HD Wt fx_table_weight(double w) {
   unsigned bad = 0;
-  Wt r = fx_weight(w, bad);
+  Wt r = fx_weight<FX_TOP>(w, bad);
   if (bad)
     r.e = FX_BAD_EXP;
   return r;
@@ -194,15 +202,11 @@ SWG_HD double fx_finish(const FxAcc &a, int P) {
   return fx_value(a.hh + (t >> 28), P);
 }
 
-// sum_j w_j x_j over N <= 14 terms; start = fx_start(sum of hi_j).
-// The result is meaningless when a word's FX_FLAG is set, which is reported
-// in `flag` (or-ed in).
+// The exponents p of N products and their largest; f: the words or-ed.
 template <int N>
-SWG_HD double fx_sum(const Wt (&w)[N], const fx_t (&x)[N], long long start,
-                     unsigned &flag) {
-  static_assert(N <= 14, "the 64-bit accumulators hold 14 products");
-  int p[N];
-  unsigned f = 0;
+SWG_HD int fx_exps(const Wt (&w)[N], const fx_t (&x)[N], int (&p)[N],
+                   unsigned &f) {
+  f = 0;
 #pragma unroll
   for (int j = 0; j < N; ++j) {
     f |= unsigned(x[j]);
@@ -212,12 +216,62 @@ SWG_HD double fx_sum(const Wt (&w)[N], const fx_t (&x)[N], long long start,
 #pragma unroll
   for (int j = 1; j < N; ++j)
     P = P > p[j] ? P : p[j];
+  return P;
+}
+
+// the largest exponent of the weights
+template <int N> SWG_HD int fx_top(const Wt (&w)[N]) {
+  int t = w[0].e;
+#pragma unroll
+  for (int j = 1; j < N; ++j)
+    t = t > w[j].e ? t : w[j].e;
+  return t;
+}
+
+// FX_FLAG where a sum without LOW is left to FP64: a flagged word, or a largest
+// exponent that may be a zero's beside a word that is not zero (without a weight
+// that is not zero the sum is, and the exponent below half FX_ZERO_EXP).
+SWG_HD unsigned fx_left(int P, int top, unsigned f) {
+  constexpr int NONE = FX_ZERO_EXP / 2;
+  if (unsigned(P - NONE) <= unsigned(top - NONE) && f != 0)
+    f = FX_FLAG;
+  return f & FX_FLAG;
+}
+
+// sum_j w_j x_j over N <= 14 terms; start = fx_start(sum of hi_j), top: no
+// weight's exponent is above it.  The result is meaningless when a word's
+// FX_FLAG is set, or without LOW where fx_left says so, which is reported in
+// `flag` (or-ed in).  LOW's branch keeps the compiler from mixing what stands
+// before and after it: k_edge_final takes 0.5 % longer with it, k_aux2 3 % and
+// k_cell_tracers with 8 tracers 8 % (630 -> 681 us at 256x256x64).
+template <int N, bool LOW>
+SWG_HD double fx_sum(const Wt (&w)[N], const fx_t (&x)[N], long long start,
+                     int top, unsigned &flag) {
+  static_assert(N <= 14, "the 64-bit accumulators hold 14 products");
+  int p[N];
+  unsigned f;
+  int P = fx_exps(w, x, p, f);
+  if (!LOW) {
+    flag |= fx_left(P, top, f);
+  } else {
+    if (P <= top && f != 0) {
+      P = FX_ZERO_EXP;
+#pragma unroll
+      for (int j = 0; j < N; ++j)
+        P = unsigned(x[j]) != 0 && p[j] > P ? p[j] : P;
+    }
+    flag |= f & FX_FLAG;
+  }
   FxAcc a{0, 0, start};
 #pragma unroll
   for (int j = 0; j < N; ++j)
     fx_mac(a, w[j], x[j], P, p[j]);
-  flag |= f & FX_FLAG;
   return fx_finish(a, P);
+}
+template <int N>
+SWG_HD double fx_sum(const Wt (&w)[N], const fx_t (&x)[N], long long start,
+                     unsigned &flag) {
+  return fx_sum<N, true>(w, x, start, fx_top(w), flag);
 }
 
 // ---- sums of float64 values as they are

@@ -182,6 +182,97 @@ def test_sum_error(lib, n, spread_w, spread_x):
         assert abs(Fraction(r) - exact) <= tol * Fraction(1001, 1000)
 
 
+@pytest.mark.parametrize("n", [7, 8, 14])
+@pytest.mark.parametrize("spread", [20, 40, 60, 100, 300])
+@pytest.mark.parametrize("zeros", [1, 3])
+def test_zeros_under_the_largest_weights(lib, n, spread, zeros):
+    """Values as small as the words hold, with weights 2^-spread and smaller,
+    beside zeros under the largest weights: the bound of test_sum_error, M
+    being the largest product that is not zero."""
+    rng = random.Random(31 * n + spread + zeros)
+    for trial in range(600):
+        w = [rng.choice((-1, 1)) * (1 + rng.random()) * 2.0**rng.randint(-2, 60)
+             if j < zeros else
+             rng.choice((-1, 1)) * (1 + rng.random())
+             * 2.0**-(spread + rng.randint(0, 9)) for j in range(n)]
+        x = [0.0 if j < zeros else rng.choice((-1, 1)) * (1 + rng.random())
+             * 2.0**rng.randint(-314, -300 + trial % 200) for j in range(n)]
+        if trial % 3 == 0:
+            x[-1] = 0.0
+        if trial % 3 == 1:
+            w[-1] = 0.0
+        order = rng.sample(range(n), n)
+        w, x = [w[j] for j in order], [x[j] for j in order]
+        r, flag = _sum(lib, w, x)
+        assert flag == 0
+        prods = [Fraction(a) * Fraction(b) for a, b in zip(w, x)]
+        exact, M = sum(prods), max(abs(p) for p in prods)
+        tol = (n * (Fraction(1, 2**56) + Fraction(1, 2**59))
+               + Fraction(1, 2**56)) * M + Fraction(1, 2**53) * abs(exact)
+        assert abs(Fraction(r) - exact) <= tol * Fraction(1001, 1000)
+
+
+LEFT_SRC = r"""
+#include "swg_fixed.cuh"
+using namespace swg;
+extern "C" double sum12(const double *w, const double *x, unsigned *flag) {
+  Wt W[12];
+  fx_t X[12];
+  long long s = 0;
+  unsigned f = 0;
+  for (int j = 0; j < 12; ++j) {
+    W[j] = fx_weight<FX_TOP>(w[j], f);
+    X[j] = fx_word(x[j]);
+    s += W[j].hi;
+  }
+  double r = fx_sum<12, false>(W, X, fx_start(s), FX_TOP, f);
+  *flag = f;
+  return r;
+}
+"""
+
+
+def test_sums_that_leave_small_products_to_fp64(tmp_path):
+    """The tracer passes' form: within the bound, or left to FP64, which no
+    sum with a product of 2^-278 and more is, nor one of zero
+    weights or values alone."""
+    src, so = tmp_path / "left.cpp", tmp_path / "left.so"
+    src.write_text(LEFT_SRC)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC,
+                    "-o", str(so), str(src)], check=True)
+    lib = ctypes.CDLL(str(so))
+    lib.sum12.restype = ctypes.c_double
+    lib.sum12.argtypes = [ctypes.POINTER(ctypes.c_double),
+                          ctypes.POINTER(ctypes.c_double),
+                          ctypes.POINTER(ctypes.c_uint)]
+    rng = random.Random(5)
+    left = 0
+    for trial in range(6000):
+        lo, wlo = (-284, -200) if trial % 2 else (-30, -40)
+        w = [rng.choice((-1, 1)) * (1 + rng.random()) * 2.0**rng.randint(wlo, 34)
+             for _ in range(12)]
+        x = [rng.choice((-1, 1)) * (1 + rng.random()) * 2.0**rng.randint(lo - 30, lo)
+             for _ in range(12)]
+        for _ in range(rng.randint(0, 8)):
+            (w if rng.random() < 0.5 else x)[rng.randrange(12)] = 0.0
+        r, flag = _sum(lib, w, x)
+        prods = [Fraction(a) * Fraction(b) for a, b in zip(w, x)]
+        exact, M = sum(prods), max(abs(p) for p in prods)
+        if flag:
+            left += 1
+            assert flag == 0x80
+            assert M < Fraction(1, 2**278)
+            continue
+        tol = (12 * (Fraction(1, 2**56) + Fraction(1, 2**59))
+               + Fraction(1, 2**56)) * M + Fraction(1, 2**53) * abs(exact)
+        assert abs(Fraction(r) - exact) <= tol * Fraction(1001, 1000)
+    assert left > 100
+    assert _sum(lib, [2.0**36] + [1.0] * 11, [1.0] * 12)[1] == 0x80
+    assert _sum(lib, [3.0] * 12, [0.0] * 12) == (0.0, 0)
+    assert _sum(lib, [0.0] * 12, [3.0, 1e-90] * 6) == (0.0, 0)
+    assert _sum(lib, [0.0] * 11 + [2.0], [1e-90] * 11 + [3.0]) == (6.0, 0)
+
+
 def _raw(lib, w, x):
     n = len(w)
     f = ctypes.c_uint()

@@ -205,3 +205,30 @@ def test_bad_weights_beside_finite_elements_in_a_batch(T, del4):
     for s, want in zip(states, single):
         for g, w in zip(s.download(), want):
             np.testing.assert_array_equal(g, w)
+
+
+@pytest.mark.parametrize("del4", [True, False])
+def test_small_products_beside_calm_edges(del4):
+    """Tracers whose products are near the words' lower end, beside zeros under
+    larger weights (calm edges of every smaller magnitude): each tracer within
+    the bound of its own scale, and updated once."""
+    cfg = (ALL if del4 else
+           dict(f0=1e-4, grav=9.81, visc_del2=1e3, visc_del4=1e9))
+    mesh, params, model, omd = build(10, 8, 33, dict(cfg, T=5))
+    h, vn, tr = state(mesh, 5, 31)
+    for j, f in enumerate((1e-20, 1e-40, 0.0, 1e-60)):
+        vn[j::5] *= f
+    tr[1] *= 1e-70
+    tr[2] *= 1e-80
+    tr[3] *= 1e-90
+    tr[1:4, ::3] = 0.0
+    S = og.ShallowWaterState(mesh, params)
+    S.upload(h, vn, tr)
+    og.LSRKStepper(model, 1).do_step(0.0, 1.0, S)
+    want = omd.step(h.copy(), vn.copy(), tr.copy(), 0.0, 1.0, 1, kind="lsrk",
+                    nstages=1)
+    got = S.download()
+    for g, w in zip(got[:2], want[:2]):
+        assert rel_diff(g, w) <= TOL
+    for g, w in zip(got[2], want[2]):
+        assert rel_diff(g, w) <= TOL
