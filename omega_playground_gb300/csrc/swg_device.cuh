@@ -879,8 +879,11 @@ __device__ __forceinline__ void pt_pv_sum(const MeshView &m, const AuxView &a,
 #pragma unroll
     for (int j = 0; j < NE; ++j) {
       const int4 s4 = __ldg(reinterpret_cast<const int4 *>(m.fxe) + NE * e + j);
+      const ulonglong2 v = reinterpret_cast<const ulonglong2 *>(
+          a.FGx)[unsigned(s4.x) * K + unsigned(k)];
       w[j] = {s4.y, s4.z, s4.w};
-      x[j] = a.FGx[2 * size_t(unsigned(s4.x) * K + unsigned(k))];
+      x[j] = v.x;
+      flag |= unsigned(v.y) & FX_FLAG; // of F Q: FP64 there takes both sums
     }
     S1 = fx_sum<NE, true>(w, x, __ldg(m.fxe0 + e), FX_TOP, flag);
   }
