@@ -404,11 +404,14 @@ int profile_read(int max_kernels, char *names, double *total_ms,
 namespace {
 
 // Whether the pairs of passes run as one launch (per-kernel timing keeps them
-// apart).
-template <class T> bool small_model(const MeshView &m, const AuxViewT<T> &a) {
+// apart).  Those sum velocities and thicknesses in FP64: a level slice of a
+// model with fixed-point sums of them (p.raw, FGx) keeps the passes apart.
+template <class T>
+bool small_model(const MeshView &m, const ModelView &p, const AuxViewT<T> &a) {
   if (!std::is_same<T, double>::value || g_profile)
     return false;
-  return !a.FGx && (long long)m.nedges * m.nlayers < SMALL_EDGE_LEVELS;
+  return !a.FGx && !p.raw &&
+         (long long)m.nedges * m.nlayers < SMALL_EDGE_LEVELS;
 }
 
 template <class T>
@@ -442,7 +445,7 @@ void launch_aux_t(const MeshView &m, const ModelView &p, const AuxViewT<T> &a,
   // that each event pair times its own kernel alone
   if (g_profile)
     fk = nullptr;
-  if (vert && cell1 && small_model<T>(m, a)) {
+  if (vert && cell1 && small_model<T>(m, p, a)) {
     if constexpr (std::is_same<T, double>::value) {
       Scope sc("k_vertex_cell1", st);
       k_vertex_cell1<<<nblocks(VK + CK, HTPB), HTPB, 0, st>>>(m, p, a, h, vn,
@@ -520,7 +523,7 @@ void launch_tendency_t(const MeshView &m, const ModelView &p,
   // The final passes are independent unless the stage updates the state in
   // place (LSRK): there the edge pass reads h, which the cell pass rewrites,
   // so the edge pass goes first.
-  if (edge && cell && s.ep.mode != EPI_LSRK && small_model<T>(m, a)) {
+  if (edge && cell && s.ep.mode != EPI_LSRK && small_model<T>(m, p, a)) {
     if constexpr (std::is_same<T, double>::value) {
       NvtxRange r("vn_tendency+h_tendency+tr_tendency");
       Scope sc("k_final", st);

@@ -260,3 +260,28 @@ def test_taped_and_recomputed_pv_sums_agree(stepper, nstages):
     for g in grads[1:]:
         for a, b in zip(g, grads[0]):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("T", [0, 2])
+def test_host_chunks_of_a_model_without_pv_words(T):
+    """One TRiSK weight out of range: the model's PV sums are FP64, its vertex
+    and divergence sums fixed-point still, and so are those of level chunks
+    small enough for the joint launches."""
+    import pyoracle
+    from test_general_mesh_gpu import TABLES, models
+    om = pyoracle.OracleMesh(40, 34, 1e4, 33)
+    t = om.tables
+    t["weights_on_edge"][7, 1] = 1e-130
+    gm = og.MPASMesh.from_tables({n: t[n] for n in TABLES}, 33)
+    _, gp, model = models(om, gm, T)
+    x = state(gm, T, 3)
+    S = og.ShallowWaterState(gm, gp)
+    S.upload(*x)
+    og.RK4Stepper(model).step(S, 0.0, 1.0, 1)
+    hs = og.HostStepper(model, "rk4", 4, 8)
+    arrs = hs.pinned_state()
+    for a, b in zip(arrs, x):
+        a[...] = b
+    hs.step(*arrs, 0.0, 1.0, 1)
+    for g, w in zip(arrs, S.download()):
+        np.testing.assert_array_equal(g, w)
