@@ -183,33 +183,22 @@ int cell_terms_table(std::vector<void *> &allocs, const MeshView &m,
   return SWG_OK;
 }
 
-// The words of the fixed-point sums: ne pairs for the fluxes, nt each for the
-// tracers and (lap) their Laplacians.  They only speed the sums up, so they
-// are left out (all null, FP64 sums) where they would take more than a
-// quarter of the free device memory: a model that fitted without them must
-// leave room for the states and steppers that come after it.  `must`: as
-// given, without that rule.
-int alloc_words(std::vector<void *> &allocs, size_t ne, size_t nt, bool lap,
-                bool must, AuxView &a) {
-  const size_t nl = lap ? nt : 0;
-  if (!must) {
-    size_t free_b = 0, total_b = 0;
-    cudaError_t err = cudaMemGetInfo(&free_b, &total_b);
-    if (err != cudaSuccess)
-      return cuda_fail(err, "cudaMemGetInfo (work arrays)");
-    if ((2 * ne + nt + nl) * sizeof(fx_t) > free_b / 4)
-      return SWG_OK;
-  }
-  double *f = nullptr, *n = nullptr, *l = nullptr;
-  if (ne)
-    TRY(dalloc(allocs, 2 * ne, &f));
-  if (nt)
-    TRY(dalloc(allocs, nt, &n));
-  if (nl)
-    TRY(dalloc(allocs, nl, &l));
-  a.FGx = reinterpret_cast<fx_t *>(f);
-  a.nx = reinterpret_cast<fx_t *>(n);
-  a.lx = reinterpret_cast<fx_t *>(l);
+// Words of the fixed-point sums (ModelView, AuxView) of a model.
+size_t words_bytes(const swg_mesh_s *m, const ModelView &p, const FxUse &fx) {
+  const size_t E = m->nedges, C = m->ncells, K = m->nlayers, T = p.ntracers;
+  return ((fx.pv ? 2 * E : 0) + (fx.tr ? (p.tr_del4 ? 2 : 1) * T * C : 0)) * K *
+         sizeof(fx_t);
+}
+// Whether a model keeps them: they only speed the sums up, so not where they
+// take more than a quarter of the device's memory, to leave room for the states
+// and steppers that come after the model.  By the sizes and the device alone,
+// not by what is free: equal models sum alike, wherever they are created.
+int keep_words(size_t bytes, bool *keep) {
+  size_t free_b = 0, total_b = 0;
+  cudaError_t err = cudaMemGetInfo(&free_b, &total_b);
+  if (err != cudaSuccess)
+    return cuda_fail(err, "cudaMemGetInfo (work arrays)");
+  *keep = bytes <= total_b / 4;
   return SWG_OK;
 }
 
@@ -677,36 +666,61 @@ extern "C" int swg_model_create_ex(swg_mesh mesh, const swg_params *p,
   const bool vn = pv.do_vn;
   const bool vdiss = vn && (pv.vel_del2 || pv.vel_del4);
   const bool v4 = vn && pv.vel_del4;
-  const FxUse fx = fx_use(mesh, pv);
+  FxUse fx = fx_use(mesh, pv);
   pv.raw = fx.raw;
-  if ((rc = alloc_words(A, fx.pv ? E * K : 0, fx.tr ? T * C * K : 0,
-                        pv.tr_del4, mesh->fx_given, a)) != SWG_OK) {
-    swg_model_destroy(md);
-    return rc;
-  }
-  struct Need {
-    bool on;
-    size_t n;
-    double **p;
-  } need[] = {
-      {vn, V * K, &a.q},        {vdiss, V * K, &a.zeta},
-      {v4, V * K, &a.z4},       {vdiss, C * K, &a.div},
-      {vn, C * K, &a.ke},       {v4, C * K, &a.d4},
-      {vn, E * K, &a.u2},
-      {T > 0, T * C * K, &a.ntr},
-      {T > 0 && pv.tr_del4, T * C * K, &a.lap},
-      {true, E * K, &a.F},      {vn && !a.FGx, E * K, &a.G},
-      // the mean thickness is kept always: the per-field tendency calls
-      // read the last auxiliary state's (the reference's m_mean_h_edge)
-      {vn, E * K, &a.Q},        {true, E * K, &a.mh},
-      {vdiss, E * K, &a.d2u},
-      {v4 && mesh->view.dv4_differs, E * K, &a.d2u4},
-  };
-  for (auto &nd : need)
-    if (!pv.linear && nd.on && (rc = dalloc(A, nd.n, nd.p))) {
+  if ((fx.pv || fx.tr) && !mesh->fx_given) {
+    bool keep = false;
+    if ((rc = keep_words(words_bytes(mesh, pv, fx), &keep))) {
       swg_model_destroy(md);
       return rc;
     }
+    fx.pv &= keep;
+    fx.tr &= keep;
+  }
+  auto alloc_work = [&](std::vector<void *> &W) {
+    a = AuxView{};
+    double *f = nullptr, *n = nullptr, *l = nullptr;
+    struct Need {
+      bool on;
+      size_t n;
+      double **p;
+    } need[] = {
+        {vn, V * K, &a.q},        {vdiss, V * K, &a.zeta},
+        {v4, V * K, &a.z4},       {vdiss, C * K, &a.div},
+        {vn, C * K, &a.ke},       {v4, C * K, &a.d4},
+        {vn, E * K, &a.u2},
+        {T > 0, T * C * K, &a.ntr},
+        {T > 0 && pv.tr_del4, T * C * K, &a.lap},
+        {true, E * K, &a.F},      {vn && !fx.pv, E * K, &a.G},
+        // the mean thickness is kept always: the per-field tendency calls
+        // read the last auxiliary state's (the reference's m_mean_h_edge)
+        {vn, E * K, &a.Q},        {true, E * K, &a.mh},
+        {vdiss, E * K, &a.d2u},
+        {v4 && mesh->view.dv4_differs, E * K, &a.d2u4},
+        {fx.pv, 2 * E * K, &f},   {fx.tr, T * C * K, &n},
+        {fx.tr && pv.tr_del4, T * C * K, &l},
+    };
+    for (auto &nd : need)
+      if (!pv.linear && nd.on)
+        TRY(dalloc(W, nd.n, nd.p));
+    a.FGx = reinterpret_cast<fx_t *>(f);
+    a.nx = reinterpret_cast<fx_t *>(n);
+    a.lx = reinterpret_cast<fx_t *>(l);
+    return int(SWG_OK);
+  };
+  std::vector<void *> work;
+  rc = alloc_work(work);
+  if (rc == SWG_ERR_OOM && (fx.pv || fx.tr) && !mesh->fx_given) {
+    // no room with the words: a slice's sums are its model's, others run in FP64
+    free_all(work);
+    fx.pv = fx.tr = false;
+    rc = alloc_work(work);
+  }
+  A.insert(A.end(), work.begin(), work.end());
+  if (rc != SWG_OK) {
+    swg_model_destroy(md);
+    return rc;
+  }
   if (!a.d2u4)
     a.d2u4 = a.d2u;
   if ((rc = dalloc(A, 1024, &md->partials)) || (rc = fork_create(md->fork))) {

@@ -285,3 +285,36 @@ def test_host_chunks_of_a_model_without_pv_words(T):
     hs.step(*arrs, 0.0, 1.0, 1)
     for g, w in zip(arrs, S.download()):
         np.testing.assert_array_equal(g, w)
+
+
+def test_equal_models_sum_alike_whatever_memory_is_free():
+    """The words are chosen by the model's size, not by the free memory: a
+    second model beside less free memory gives the first one's bits.  Where the
+    words do not fit at all the model runs in FP64, within the parity bound."""
+    import torch
+    T, mb = 8, 1 << 20
+    mesh, params, model, _ = build(128, 128, 64, dict(ALL, T=T))
+    S, D = og.ShallowWaterState(mesh, params), og.ShallowWaterState(mesh, params)
+    S.upload(*state(mesh, T, 31))
+    model.compute_tendency(D, S, 0.0)
+    want = D.download()
+    cl = 8 * mesh.m_ncells * mesh.m_nlayers
+    words, rest = 22 * cl, 43 * cl  # of both fluxes, 8 tracers and Laplacians
+
+    def with_free(nbytes):
+        torch.cuda.empty_cache()
+        fill = torch.empty(torch.cuda.mem_get_info()[0] - nbytes,
+                           dtype=torch.uint8, device="cuda")
+        other = og.ShallowWaterModel(mesh, params)
+        other.compute_tendency(D, S, 0.0)
+        got = D.download()
+        del other, fill
+        torch.cuda.empty_cache()
+        return got
+
+    for g, w in zip(with_free(3 * words + 64 * mb), want):
+        np.testing.assert_array_equal(g, w)
+    for g, w in zip(with_free(rest + 96 * mb), want):
+        assert rel_diff(g, w) <= TOL
+    for g, w in zip(with_free(8 * (words + rest)), want):
+        np.testing.assert_array_equal(g, w)
