@@ -78,6 +78,12 @@ int dalloc(std::vector<void *> &allocs, size_t n, double **dev) {
   return SWG_OK;
 }
 
+void free_all(std::vector<void *> &allocs) {
+  for (void *p : allocs)
+    cudaFree(p);
+  allocs.clear();
+}
+
 int check_launch(const char *what) {
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? SWG_OK : cuda_fail(err, what);
@@ -106,24 +112,47 @@ __global__ void k_cell_terms(MeshView m, const double *r4, FxSlot *out) {
   if (i < 6LL * m.ncells)
     out[i] = FxSlot{m.nbc[i], fx_table_weight(r4[i])};
 }
-// mv.fxe, mv.fxe0: left null when a weight is out of range
+// Tables of terms only speed sums up: `make` fills the allocations T and
+// reports weights out of range in *bad.  They are kept (allocs) when there is
+// memory for them and every weight is in range; otherwise *kept is false.
+template <class F>
+int optional_tables(std::vector<void *> &allocs, const F &make, bool *kept) {
+  std::vector<void *> T;
+  double *b = nullptr;
+  unsigned bad = 0;
+  int rc = dalloc(T, 1, &b);
+  if (rc == SWG_OK)
+    rc = make(T, reinterpret_cast<unsigned *>(b));
+  if (rc == SWG_OK) {
+    cudaError_t err = cudaMemcpy(&bad, b, sizeof(bad), cudaMemcpyDeviceToHost);
+    if (err != cudaSuccess)
+      rc = cuda_fail(err, "tables of fixed-point terms");
+  }
+  *kept = rc == SWG_OK && !bad;
+  if (*kept)
+    allocs.insert(allocs.end(), T.begin(), T.end());
+  else
+    free_all(T);
+  return rc == SWG_ERR_OOM ? int(SWG_OK) : rc;
+}
+// mv.fxe, mv.fxe0
 int edge_terms_table(std::vector<void *> &allocs, MeshView &mv, int ne) {
-  double *t = nullptr, *s = nullptr, *b = nullptr;
-  TRY(dalloc(allocs, size_t(ne) * mv.nedges * (sizeof(FxSlot) / 8), &t));
-  TRY(dalloc(allocs, mv.nedges, &s));
-  TRY(dalloc(allocs, 1, &b));
-  FxSlot *slots = reinterpret_cast<FxSlot *>(t);
-  long long *start = reinterpret_cast<long long *>(s);
-  unsigned *bad = reinterpret_cast<unsigned *>(b), bad_h = 0;
-  k_edge_terms<<<unsigned((mv.nedges + 255) / 256), 256>>>(mv, ne, slots,
-                                                           start, bad);
-  TRY(check_launch("edge terms table"));
-  cudaError_t err = cudaMemcpy(&bad_h, bad, 4, cudaMemcpyDeviceToHost);
-  if (err != cudaSuccess)
-    return cuda_fail(err, "edge terms table");
-  if (!bad_h) {
-    mv.fxe = slots;
-    mv.fxe0 = start;
+  double *t = nullptr, *s = nullptr;
+  bool kept = false;
+  TRY(optional_tables(
+      allocs,
+      [&](std::vector<void *> &T, unsigned *bad) {
+        TRY(dalloc(T, size_t(ne) * mv.nedges * (sizeof(FxSlot) / 8), &t));
+        TRY(dalloc(T, mv.nedges, &s));
+        k_edge_terms<<<unsigned((mv.nedges + 255) / 256), 256>>>(
+            mv, ne, reinterpret_cast<FxSlot *>(t),
+            reinterpret_cast<long long *>(s), bad);
+        return check_launch("edge terms table");
+      },
+      &kept));
+  if (kept) {
+    mv.fxe = reinterpret_cast<FxSlot *>(t);
+    mv.fxe0 = reinterpret_cast<long long *>(s);
   }
   return SWG_OK;
 }
@@ -137,7 +166,7 @@ __global__ void k_raw_terms(const int *idx, const double *w, long long n,
   if (flag)
     atomicOr(bad, flag);
 }
-// mv.cvx, kvx, cdx: left null when a weight is out of range
+// mv.cvx, kvx, cdx
 int raw_terms_tables(std::vector<void *> &allocs, MeshView &mv) {
   const long long V3 = 3LL * mv.nvertices, C6 = 6LL * mv.ncells;
   struct {
@@ -145,26 +174,28 @@ int raw_terms_tables(std::vector<void *> &allocs, MeshView &mv) {
     const double *w;
     long long n;
     const FxSlot **out;
-  } tab[] = {{mv.ev, mv.cvr, V3, &mv.cvx},
-             {mv.cv, mv.kvh, V3, &mv.kvx},
-             {mv.ec, mv.ccd, C6, &mv.cdx}};
-  double *b = nullptr;
-  TRY(dalloc(allocs, 1, &b));
-  unsigned *bad = reinterpret_cast<unsigned *>(b), bad_h = 0;
-  FxSlot *slots[3];
-  for (int t = 0; t < 3; ++t) {
-    double *d = nullptr;
-    TRY(dalloc(allocs, size_t(tab[t].n) * (sizeof(FxSlot) / 8), &d));
-    slots[t] = reinterpret_cast<FxSlot *>(d);
-    k_raw_terms<<<unsigned((tab[t].n + 255) / 256), 256>>>(
-        tab[t].idx, tab[t].w, tab[t].n, slots[t], bad);
-    TRY(check_launch("raw terms table"));
-  }
-  cudaError_t err = cudaMemcpy(&bad_h, bad, 4, cudaMemcpyDeviceToHost);
-  if (err != cudaSuccess)
-    return cuda_fail(err, "raw terms table");
-  for (int t = 0; t < 3 && !bad_h; ++t)
-    *tab[t].out = slots[t];
+    FxSlot *slots;
+  } tab[] = {{mv.ev, mv.cvr, V3, &mv.cvx, nullptr},
+             {mv.cv, mv.kvh, V3, &mv.kvx, nullptr},
+             {mv.ec, mv.ccd, C6, &mv.cdx, nullptr}};
+  bool kept = false;
+  TRY(optional_tables(
+      allocs,
+      [&](std::vector<void *> &T, unsigned *bad) {
+        for (auto &t : tab) {
+          double *d = nullptr;
+          TRY(dalloc(T, size_t(t.n) * (sizeof(FxSlot) / 8), &d));
+          t.slots = reinterpret_cast<FxSlot *>(d);
+          k_raw_terms<<<unsigned((t.n + 255) / 256), 256>>>(t.idx, t.w, t.n,
+                                                            t.slots, bad);
+          TRY(check_launch("raw terms table"));
+        }
+        return int(SWG_OK);
+      },
+      &kept));
+  for (auto &t : tab)
+    if (kept)
+      *t.out = t.slots;
   return SWG_OK;
 }
 int cell_terms_table(std::vector<void *> &allocs, const MeshView &m,
@@ -200,12 +231,6 @@ int keep_words(size_t bytes, bool *keep) {
     return cuda_fail(err, "cudaMemGetInfo (work arrays)");
   *keep = bytes <= total_b / 4;
   return SWG_OK;
-}
-
-void free_all(std::vector<void *> &allocs) {
-  for (void *p : allocs)
-    cudaFree(p);
-  allocs.clear();
 }
 
 bool in_range(const int *a, size_t n, int lo, int hi) {
@@ -423,8 +448,8 @@ extern "C" int swg_mesh_create(const swg_mesh_desc *d, swg_mesh *out) try {
       (rc = upload(A, inv_dv4.data(), E, &mv.inv_dv4)) ||
       (rc = upload(A, eoe.data(), size_t(NE) * E, &mv.eoe)) ||
       (rc = upload(A, woe.data(), size_t(NE) * E, &mv.woe)) ||
-      (rc = edge_terms_table(A, mv, NE)) ||
-      (rc = raw_terms_tables(A, mv)) ||
+      (fx_large(mv) && (rc = edge_terms_table(A, mv, NE))) ||
+      (fx_large(mv) && (rc = raw_terms_tables(A, mv))) ||
       (rc = upload(A, m->scale2_h.data(), E, &mv.scale2)) ||
       (rc = upload(A, m->scale4_h.data(), E, &mv.scale4)) ||
       (rc = upload(A, d->area_cell, C, &mv.area_cell_d)) ||
@@ -657,7 +682,6 @@ extern "C" int swg_model_create_ex(swg_mesh mesh, const swg_params *p,
       (rc = upload(A, kd2.data(), 6 * C, &pv.kd2)) ||
       (rc = upload(A, r4.data(), 6 * C, &pv.r4)) ||
       (rc = upload(A, r4s.data(), C, &pv.r4sum)) ||
-      (T > 0 && pv.tr_del4 && (rc = cell_terms_table(A, mesh->view, pv))) ||
       (!r4f.empty() && (rc = upload(A, r4f.data(), C, &pv.r4f)))) {
     swg_model_destroy(md);
     return rc;
@@ -679,6 +703,7 @@ extern "C" int swg_model_create_ex(swg_mesh mesh, const swg_params *p,
   }
   auto alloc_work = [&](std::vector<void *> &W) {
     a = AuxView{};
+    pv.r4x = nullptr;
     double *f = nullptr, *n = nullptr, *l = nullptr;
     struct Need {
       bool on;
@@ -706,6 +731,8 @@ extern "C" int swg_model_create_ex(swg_mesh mesh, const swg_params *p,
     a.FGx = reinterpret_cast<fx_t *>(f);
     a.nx = reinterpret_cast<fx_t *>(n);
     a.lx = reinterpret_cast<fx_t *>(l);
+    if (a.lx)
+      TRY(cell_terms_table(W, mesh->view, pv));
     return int(SWG_OK);
   };
   std::vector<void *> work;

@@ -353,14 +353,19 @@ constexpr long long SMALL_EDGE_LEVELS = 1 << 16;
 // with more tracers the first cell pass is bound by their memory traffic, not
 // by the divergence's FP64 (8 tracers, 256x256x64: 149 us in FP64, 154 fixed)
 constexpr int FX_MAX_DIV_TRACERS = 4;
+// whether models of the mesh may have fixed-point PV, vertex and divergence
+// sums, and so whether it keeps their tables
+inline bool fx_large(const MeshView &m) {
+  return m.nlayers >= FX_MIN_LEVELS &&
+         (long long)m.nedges * m.nlayers >= FX_MIN_EDGE_LEVELS;
+}
 inline FxUse fx_use(const swg_mesh_s *mesh, const ModelView &p) {
   if (p.linear)
     return {false, false, 0};
   if (mesh->fx_given)
     return mesh->fx;
   const bool levels = mesh->nlayers >= FX_MIN_LEVELS;
-  const bool large =
-      levels && (long long)mesh->nedges * mesh->nlayers >= FX_MIN_EDGE_LEVELS;
+  const bool large = fx_large(mesh->view);
   return {large && p.do_vn && mesh->view.fxe,
           levels && p.ntracers > 0 &&
               (p.tr_del4 || p.ntracers >= FX_MIN_TRACERS),

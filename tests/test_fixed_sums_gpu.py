@@ -318,3 +318,39 @@ def test_equal_models_sum_alike_whatever_memory_is_free():
         assert rel_diff(g, w) <= TOL
     for g, w in zip(with_free(8 * (words + rest)), want):
         np.testing.assert_array_equal(g, w)
+
+
+def _mesh_bytes(nx, K, edit=None):
+    """Device memory of a mesh's tables."""
+    import torch
+    from test_general_mesh_gpu import TABLES
+    h = og.PlanarHexagonalMesh(nx, nx, 1e4, K)
+    t = {n: np.array(h.tables[n]) for n in TABLES}
+    if edit:
+        edit(t)
+    del h
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    gm = og.MPASMesh.from_tables(t, K)
+    assert gm.handle
+    return before - torch.cuda.mem_get_info()[0]
+
+
+def test_tables_are_kept_only_where_they_are_read():
+    """The tables of the fixed-point sums (about 700 B per cell): not on a
+    mesh of one level or below the size rule, nor with a weight they cannot
+    hold."""
+    cells, mb = 300 * 300, 1 << 20
+    one = _mesh_bytes(300, 1)
+    large = _mesh_bytes(300, 2)
+    assert large - one >= 600 * cells
+    small = _mesh_bytes(64, 8)  # below 2^17 edge-levels
+    assert small <= one * 64 * 64 / cells + 32 * mb
+
+    def edit(t):
+        t["weights_on_edge"][7, 1] = 1e-130
+        t["area_triangle"][5] *= 1e-70
+
+    rejected = _mesh_bytes(300, 2, edit)
+    # ten weights an edge instead of eight where the edit adds a ninth
+    assert rejected - one <= 24 * 3 * cells + 8 * mb
