@@ -491,14 +491,7 @@ void adj_tendency(swg_adjoint ad, const double *h, const double *vn,
                   cudaStream_t st) {
   swg_model md = ad->model;
   launch_aux(md->mesh->view, md->view, md->aux, h, vn, tr, st, &md->fork);
-  // fixed-point PV sums go to the edge pass's own work array: each thread
-  // reads its S1 before it writes that element of lQ
-  AuxView aux = md->aux;
-  if (aux.FGx && !md->view.off_pv) {
-    aux.S1 = ad->aw.lQ;
-    launch_pv_sum(md->mesh->view, aux, st);
-  }
-  AdjIO io{};
+  AdjIO io{}; // no tape: the edge pass forms the PV sum itself
   io.h = h;
   io.vn = vn;
   io.tr = tr;
@@ -508,7 +501,7 @@ void adj_tendency(swg_adjoint ad, const double *h, const double *vn,
   io.lh = out->h;
   io.lvn = out->vn;
   io.ltr = out->tr;
-  adj_passes(ad, aux, io, st);
+  adj_passes(ad, md->aux, io, st);
 }
 
 void lincomb(swg_state y, swg_state x1, swg_state x2, double a, double b,

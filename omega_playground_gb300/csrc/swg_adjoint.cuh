@@ -199,8 +199,8 @@ static __device__ __noinline__ double vertex_rcp(const MeshView &m, const double
   return rcp_nr(hv);
 }
 
-// the PV flux sum S1 = sum_j w_j F_j of edge e, level k, in FP64 (a model with
-// fixed-point sums has it in S1: pt_pv_sum)
+// the PV flux sum S1 = sum_j w_j F_j of edge e, level k, in FP64 (tapes of a
+// model with fixed-point sums have it in S1: pt_pv_sum)
 template <int NE>
 __device__ __noinline__ double s1_of(const MeshView &m, const AuxView &a,
                                      int e, int k) {
@@ -333,7 +333,6 @@ pa_edge(const MeshView &m, const ModelView &p, const AuxView &a,
         lG = fma(ws, io.mvn[is], lG);
         lFq = fma(ws, w.Qmu[is], lFq);
       }
-      // (S1 may be lQ itself, see adj_tendency)
       const double S1 = a.S1 ? a.S1[i] : s1_of<NE>(m, a, e, k);
       w.lQ[i] = fma(S1, mu, mul_reg(F, lG));
       lF = fma(a.Q[i], lG, lFq);

@@ -354,3 +354,29 @@ def test_tables_are_kept_only_where_they_are_read():
     rejected = _mesh_bytes(300, 2, edit)
     # ten weights an edge instead of eight where the edit adds a ninth
     assert rejected - one <= 24 * 3 * cells + 8 * mb
+
+
+def test_a_tendency_gradient_launches_no_pass_for_the_pv_sums():
+    """One gradient of one tendency has no tape to fill: its launches are the
+    same on either side of the size rule, and the dot product with the
+    tangent-linear model holds."""
+    counts = []
+    for K in (32, 33):
+        mesh, params, model, _ = build(40, 34, K, dict(ALL, T=2))
+        adj = og.Adjoint(model, 1)
+        x, dx, mu, lam, jd = (og.ShallowWaterState(mesh, params)
+                              for _ in range(5))
+        x.upload(*state(mesh, 2, 31))
+        d, m = state(mesh, 2, 41), state(mesh, 2, 51)
+        d = d[0] - 1000.0, 0.1 * d[1], d[2] - 1000.0
+        m = m[0] - 1000.0, m[1], 1e-3 * m[2]
+        dx.upload(*d)
+        mu.upload(*m)
+        n = og.kernel_launches()
+        adj.adj_tendency(x, mu, lam)
+        counts.append(og.kernel_launches() - n)
+        adj.tlm_tendency(x, dx, jd)
+        lhs = sum(float(np.sum(a * b)) for a, b in zip(jd.download(), m))
+        rhs = sum(float(np.sum(a * b)) for a, b in zip(lam.download(), d))
+        assert abs(lhs - rhs) <= 1e-12 * max(abs(lhs), abs(rhs))
+    assert counts[0] == counts[1]
