@@ -156,13 +156,18 @@ int edge_terms_table(std::vector<void *> &allocs, MeshView &mv, int ne) {
   }
   return SWG_OK;
 }
+// nslot: slots of an entity; with MAXE a zero weight is out of range too, unless
+// it is padding (the entity's first edge again)
 __global__ void k_raw_terms(const int *idx, const double *w, long long n,
-                            FxSlot *out, unsigned *bad) {
+                            int nslot, FxSlot *out, unsigned *bad) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n)
     return;
   unsigned flag = 0;
   out[i] = FxSlot{idx[i], fx_raw_weight(w[i], flag)};
+  if (nslot == MAXE && w[i] == 0.0 &&
+      (i % MAXE == 0 || idx[i] != idx[i - i % MAXE]))
+    flag |= FX_FLAG;
   if (flag)
     atomicOr(bad, flag);
 }
@@ -173,11 +178,12 @@ int raw_terms_tables(std::vector<void *> &allocs, MeshView &mv) {
     const int *idx;
     const double *w;
     long long n;
+    int nslot;
     const FxSlot **out;
     FxSlot *slots;
-  } tab[] = {{mv.ev, mv.cvr, V3, &mv.cvx, nullptr},
-             {mv.cv, mv.kvh, V3, &mv.kvx, nullptr},
-             {mv.ec, mv.ccd, C6, &mv.cdx, nullptr}};
+  } tab[] = {{mv.ev, mv.cvr, V3, 3, &mv.cvx, nullptr},
+             {mv.cv, mv.kvh, V3, 3, &mv.kvx, nullptr},
+             {mv.ec, mv.ccd, C6, MAXE, &mv.cdx, nullptr}};
   bool kept = false;
   TRY(optional_tables(
       allocs,
@@ -186,8 +192,8 @@ int raw_terms_tables(std::vector<void *> &allocs, MeshView &mv) {
           double *d = nullptr;
           TRY(dalloc(T, size_t(t.n) * (sizeof(FxSlot) / 8), &d));
           t.slots = reinterpret_cast<FxSlot *>(d);
-          k_raw_terms<<<unsigned((t.n + 255) / 256), 256>>>(t.idx, t.w, t.n,
-                                                            t.slots, bad);
+          k_raw_terms<<<unsigned((t.n + 255) / 256), 256>>>(
+              t.idx, t.w, t.n, t.nslot, t.slots, bad);
           TRY(check_launch("raw terms table"));
         }
         return int(SWG_OK);

@@ -380,3 +380,26 @@ def test_a_tendency_gradient_launches_no_pass_for_the_pv_sums():
         rhs = sum(float(np.sum(a * b)) for a, b in zip(lam.download(), d))
         assert abs(lhs - rhs) <= 1e-12 * max(abs(lhs), abs(rhs))
     assert counts[0] == counts[1]
+
+
+def test_not_finite_under_a_zero_kite_area():
+    """A thickness that is not finite reaches the potential vorticity of a
+    vertex through a kite area of zero too (0 x is NaN in FP64)."""
+    from test_general_mesh_gpu import TABLES, models
+    import pyoracle
+    om = pyoracle.OracleMesh(40, 34, 1e4, 33)
+    t = om.tables
+    t["kiteareas_on_vertex"][::2, 1] = 0.0
+    gm = og.MPASMesh.from_tables({n: t[n] for n in TABLES}, 33)
+    _, gp, model = models(om, gm, 0)
+    h, vn, _ = state(gm, 0, 3)
+    h[55, 5], h[700, 9] = np.nan, np.inf
+    S, D = og.ShallowWaterState(gm, gp), og.ShallowWaterState(gm, gp)
+    S.upload(h, vn)
+    model.compute_tendency(D, S, 0.0)
+    q = model.aux("q_vertex").reshape(gm.m_nvertices, 33)
+    k, cv = t["kiteareas_on_vertex"], t["cells_on_vertex"]
+    with np.errstate(invalid="ignore"):
+        hv = sum(k[:, j, None] * h[cv[:, j]] for j in range(3))
+    assert (~np.isfinite(hv)).any(axis=1)[::2].any()
+    np.testing.assert_array_equal(np.isnan(q), ~np.isfinite(hv))
