@@ -403,3 +403,68 @@ def test_not_finite_under_a_zero_kite_area():
         hv = sum(k[:, j, None] * h[cv[:, j]] for j in range(3))
     assert (~np.isfinite(hv)).any(axis=1)[::2].any()
     np.testing.assert_array_equal(np.isnan(q), ~np.isfinite(hv))
+
+
+def _beyond(mesh, T, seed, bad=None):
+    """A state with magnitudes beyond the words, and some values `bad`."""
+    h, vn, tr = state(mesh, T, seed)
+    tr[1] *= 1e-100
+    tr[2, ::2] = 0.0
+    tr[2, 1::4] *= 1e-97
+    vn[::3] = 0.0
+    vn[1::7] *= 1e-99
+    if bad is not None:
+        tr[0, 7, 3] = bad
+        vn[11, 2] = bad
+    return h, vn, tr
+
+
+@pytest.mark.parametrize("bad", [None, np.nan])
+@pytest.mark.parametrize("shape,K", [((10, 8), 33), ((24, 20), 37)])
+def test_noalloc_tendency_beyond_the_words(shape, K, bad):
+    from test_zz_no_alloc import _noalloc
+    mesh, params, model, _ = build(*shape, K, dict(ALL, T=3))
+    S, A, B = (og.ShallowWaterState(mesh, params) for _ in range(3))
+    S.upload(*_beyond(mesh, 3, 31, bad))
+    model.compute_tendency(A, S, 0.0)
+    assert _noalloc(mesh, params, S, B) == 0
+    og.sync()
+    want, got = A.download(), B.download()
+    for g, w in zip([*got[:2], *got[2]], [*want[:2], *want[2]]):
+        fine = np.isfinite(w)
+        np.testing.assert_array_equal(np.isfinite(g), fine)
+        assert rel_diff(np.where(fine, g, 0), np.where(fine, w, 0)) <= TOL
+
+
+@pytest.mark.parametrize("shape,K", [((10, 8), 33), ((40, 34), 33)])
+def test_taped_steps_beyond_the_words(shape, K):
+    """Adjoints of such states: an ensemble's members bitwise equal to single
+    adjoints, the taped forward bitwise equal to the plain stepper."""
+    members, want = [], []
+    for i in range(3):
+        mesh, params, model, _ = build(*shape, K - i, dict(ALL, T=3))
+        x, mu = _beyond(mesh, 3, 31 + i), state(mesh, 3, 51 + i)
+        adj = og.Adjoint(model, 2)
+        S, F, L, P = (og.ShallowWaterState(mesh, params) for _ in range(4))
+        S.upload(*x)
+        P.upload(*x)
+        L.upload(*mu)
+        adj.forward(S, 0.0, 1.0, 4, F)
+        adj.backward(L)
+        og.RK4Stepper(model).step(P, 0.0, 1.0, 4)
+        for g, w in zip(F.download(), P.download()):
+            np.testing.assert_array_equal(g, w)
+        want.append((F.download(), L.download()))
+        members.append((model, adj, S, F, L, x, mu))
+    ens = og.AdjointEnsemble([m[1] for m in members])
+    for _, _, S, _, L, x, mu in members:
+        S.upload(*x)
+        L.upload(*mu)
+    ens.forward([m[2] for m in members], 0.0, 1.0, 4, [m[3] for m in members])
+    ens.backward([m[4] for m in members])
+    og.sync()
+    for m, w in zip(members, want):
+        for got, ref in zip((m[3].download(), m[4].download()), w):
+            for g, r in zip(got, ref):
+                assert np.isfinite(r).all()
+                np.testing.assert_array_equal(g, r)
