@@ -248,9 +248,7 @@ __device__ __forceinline__ double raw_sum(const FxSlot *tab, const double *x,
     w[j] = {t.y, t.z, t.w};
     v[j] = x[unsigned(t.x) * K + k];
   }
-  // zeros of the cells' tables are padding, slots of an edge the cell has
-  // (k_raw_terms)
-  return fx_raw_sum<N, N != MAXE>(w, v, slow);
+  return fx_raw_sum(w, v, slow);
 }
 // the same in FP64, for terms the fixed-point sum leaves to it (out of line:
 // see times_rare)

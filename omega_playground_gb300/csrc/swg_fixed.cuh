@@ -297,17 +297,15 @@ SWG_HD Wt fx_raw_weight(double w, unsigned &flag) {
   return r;
 }
 
-// sum_j w_j x_j; sets `slow` when it has to be evaluated in FP64.  ZEROS: some
-// weights may be zero, and values under them that are not finite count too.
-template <int N, bool ZEROS = true>
+// sum_j w_j x_j; sets `slow` when it has to be evaluated in FP64 (a value that is
+// not finite under a zero weight does not: the tables have none but padding)
+template <int N>
 SWG_HD double fx_raw_sum(const Wt (&w)[N], const double (&x)[N], bool &slow) {
   static_assert(N <= 7, "the sum of hi in 32 bits");
-  int p[N], P = FXR_ZERO, sum = 0, top = 0;
+  int p[N], P = FXR_ZERO, sum = 0;
 #pragma unroll
   for (int j = 0; j < N; ++j) {
-    const int e = int(unsigned(fx_bits(x[j]) >> 32) & 0x7ff00000u);
-    top = top > e ? top : e;
-    p[j] = e + w[j].e;
+    p[j] = int(unsigned(fx_bits(x[j]) >> 32) & 0x7ff00000u) + w[j].e;
     P = P > p[j] ? P : p[j];
     sum += w[j].hi;
   }
@@ -329,8 +327,7 @@ SWG_HD double fx_raw_sum(const Wt (&w)[N], const double (&x)[N], bool &slow) {
     fx_mad(a.m1, w[j].hi, xl);
     fx_mad(a.m2, w[j].lo, xh);
   }
-  slow = slow || unsigned(P) - (200u << 20) >= (1535u << 20) ||
-         (ZEROS && top == 0x7ff00000);
+  slow = slow || unsigned(P) - (200u << 20) >= (1535u << 20);
   const long long t = a.m2 + (a.m1 >> 4);
   const long long R = a.hh + (t >> 28);
 #ifdef __CUDA_ARCH__

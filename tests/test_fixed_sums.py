@@ -331,13 +331,3 @@ def test_raw_sum_leaves_the_rest_to_fp64(lib):
     assert _raw(lib, [2.0**-121] + [1.0] * 5, one)[1]
     assert _raw(lib, [0.0, 0.0, 2.0], [math.pi, 1.0, 3.0]) == (6.0, 0)
     assert _raw(lib, [1.0] * 3, [0.0, -0.0, 3.0]) == (3.0, 0)
-
-
-def test_raw_sum_keeps_what_is_not_finite_under_a_zero_weight(lib):
-    """0 x is NaN where x is not finite, so FP64 has that sum too (a zero kite
-    area of a culled mesh refers to a cell all the same)."""
-    for bad in (math.inf, -math.inf, math.nan):
-        for j in range(3):
-            w, x = [1.0, 2.0, 3.0], [1.5, 2.5, 3.5]
-            w[j], x[j] = 0.0, bad
-            assert _raw(lib, w, x)[1]
