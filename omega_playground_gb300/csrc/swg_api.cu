@@ -98,12 +98,19 @@ __global__ void k_edge_terms(MeshView m, int ne, FxSlot *out, long long *start,
     return;
   long long sum = 0;
   unsigned flag = 0;
+  int lo = FX_BAD_EXP, hi = FX_ZERO_EXP; // of the weights that are not zero
   for (int j = 0; j < ne; ++j) {
-    const FxSlot t{m.eoe[ne * e + j], fx_weight<FX_TOP>(m.woe[ne * e + j], flag)};
+    const FxSlot t{m.eoe[ne * e + j], fx_weight(m.woe[ne * e + j], flag)};
     out[ne * e + j] = t;
     sum += t.w.hi;
+    if (t.w.e != FX_ZERO_EXP) {
+      lo = min(lo, t.w.e);
+      hi = max(hi, t.w.e);
+    }
   }
   start[e] = fx_start(sum);
+  if (hi - lo > FX_PV_SPREAD) // (see FxZeros; negative without weights)
+    flag |= FX_FLAG;
   if (flag)
     atomicOr(bad, flag);
 }

@@ -336,7 +336,8 @@ __device__ __forceinline__ void store_pv(const AuxViewT<T> &a, unsigned i, T F,
   if constexpr (std::is_same<T, double>::value)
     if (a.FGx) {
       reinterpret_cast<ulonglong2 *>(a.FGx)[i] =
-          make_ulonglong2(fx_word(F), fx_word(mul_reg(F, Q)));
+          make_ulonglong2(fx_word<FX_PV_MINQ>(F),
+                          fx_word<FX_PV_MINQ>(mul_reg(F, Q)));
       return;
     }
   a.G[i] = mul_reg(F, Q);
@@ -597,7 +598,7 @@ __device__ __forceinline__ void pt_aux2(const MeshView &m, const ModelView &p,
           for (int j = 0; j <= MAXE; ++j)
             x[j] = n[off[j]];
           const double L =
-              fx_sum<MAXE + 1, false>(W, x, start, FX_TOP, redo);
+              fx_sum<MAXE + 1, FX_LEAVE>(W, x, start, FX_TOP, redo);
           a.lap[base + i] = L;
           a.lx[base + i] = fx_word(L);
         }
@@ -809,8 +810,8 @@ edge_final_fixed(const MeshView &m, const ModelView &p, const AuxView &a,
     if (EARLY)
       flag = unsigned(x[0]) & FX_FLAG;
     if (!EARLY || !flag) {
-      S1 = fx_sum<NE, true>(w, x, start, FX_TOP, flag);
-      const double S2 = fx_sum<NE, true>(w, y, start, FX_TOP, flag);
+      S1 = fx_sum<NE, FX_NONE>(w, x, start, FX_TOP, flag);
+      const double S2 = fx_sum<NE, FX_NONE>(w, y, start, FX_TOP, flag);
       t = add_rn(fma(Q, S1, S2), t);
     }
   }
@@ -885,7 +886,7 @@ __device__ __forceinline__ void pt_pv_sum(const MeshView &m, const AuxView &a,
       x[j] = v.x;
       flag |= unsigned(v.y) & FX_FLAG; // of F Q: FP64 there takes both sums
     }
-    S1 = fx_sum<NE, true>(w, x, __ldg(m.fxe0 + e), FX_TOP, flag);
+    S1 = fx_sum<NE, FX_NONE>(w, x, __ldg(m.fxe0 + e), FX_TOP, flag);
   }
   if (flag) {
     S1 = 0;
@@ -999,7 +1000,7 @@ tracer_sums(const MeshView &m, const ModelView &p, const AuxView &a,
       in = epilogue_in(s.ep, s.ftr, base + off[MAXE]);
     }
     unsigned flag = 0;
-    double acc = fma(wc, nc, fx_sum<N, false>(W, x, start, FX_TOP, flag));
+    double acc = fma(wc, nc, fx_sum<N, FX_LEAVE>(W, x, start, FX_TOP, flag));
     if (D4)
       acc = fma(rc, Lc, acc);
     redo |= flag;

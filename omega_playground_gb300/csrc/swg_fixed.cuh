@@ -29,10 +29,13 @@
 //
 // A zero has no exponent: its word gives the product the exponent e_j of its
 // weight alone, which could shift smaller products out (2^-314 of that weight
-// and less).  Where the largest exponent is no more than a bound `top` of the
-// e_j and some word is not zero, the sum leaves the zeros' exponents out (LOW),
-// or it is left to FP64 with those below.  The passes take weights below 2^36
-// and the constant FX_TOP: only sums with M below 2^-278 are looked at again.
+// and less).  Three ways around it (FxZeros): where the largest exponent is no
+// more than a bound `top` of the e_j and some word is not zero, the sum leaves
+// the zeros' exponents out, or it is left to FP64 with those below; or it
+// cannot happen, with weights that lie within FX_PV_SPREAD binades of each
+// other and words of values not so small (fx_word<FX_PV_MINQ>).  The passes
+// take weights below 2^36 and the constant FX_TOP: only sums with M below
+// 2^-278 are looked at again.
 //
 // A term that cannot be represented (a flagged word, or a weight out of
 // range) makes the caller evaluate that one sum in FP64 instead: infinities
@@ -55,6 +58,8 @@ constexpr unsigned FX_FLAG = 0x80; // low-byte bit of an unrepresentable value
 constexpr int FX_ZERO_EXP = -100000; // exponent of a zero weight
 constexpr int FX_BAD_EXP = 100000;   // and of a table's out-of-range weight
 constexpr int FX_TOP = -20;          // largest exponent of a pass's weight
+constexpr int FX_PV_MINQ = 8;        // smallest q of a word of the PV sums, and
+constexpr int FX_PV_SPREAD = 3 * FX_PV_MINQ - 1; // what their weights differ by
 constexpr int FX_SCALE = -317;       // 60 - 377: result exponent offset
 
 struct Wt {
@@ -111,8 +116,8 @@ template <int TOP = 345> SWG_HD Wt fx_weight(double w, unsigned &flag) {
   return r;
 }
 
-// The word of the value x.
-SWG_HD fx_t fx_word(double x) {
+// The word of the value x; MINQ: values with a smaller q are flagged.
+template <int MINQ = 1> SWG_HD fx_t fx_word(double x) {
   const fx_t b = fx_bits(x);
   const unsigned eo = (unsigned(b >> 52) & 0x7ff) - 709u;
   const unsigned q = (eo * 21846u) >> 16; // eo / 3 for eo <= 380
@@ -122,7 +127,8 @@ SWG_HD fx_t fx_word(double x) {
                             << ((8 + r) & 63));
   X = (X ^ s) - s;
   fx_t w = fx_t(X) | (q + 1);
-  if (eo > 380u)
+  constexpr unsigned LEAST = 3 * (MINQ - 1);
+  if (eo - LEAST > 380u - LEAST)
     w = fx_is_zero(b) ? 0 : 0xff;
   return w;
 }
@@ -228,7 +234,7 @@ template <int N> SWG_HD int fx_top(const Wt (&w)[N]) {
   return t;
 }
 
-// FX_FLAG where a sum without LOW is left to FP64: a flagged word, or a largest
+// FX_FLAG where a sum with FX_LEAVE is left to FP64: a flagged word, or a largest
 // exponent that may be a zero's beside a word that is not zero (without a weight
 // that is not zero the sum is, and the exponent below half FX_ZERO_EXP).
 SWG_HD unsigned fx_left(int P, int top, unsigned f) {
@@ -238,40 +244,46 @@ SWG_HD unsigned fx_left(int P, int top, unsigned f) {
   return f & FX_FLAG;
 }
 
+// What a sum does about zeros under large weights (see above).
+enum FxZeros { FX_RESOLVE, FX_LEAVE, FX_NONE };
+
 // sum_j w_j x_j over N <= 14 terms; start = fx_start(sum of hi_j), top: no
 // weight's exponent is above it.  The result is meaningless when a word's
-// FX_FLAG is set, or without LOW where fx_left says so, which is reported in
-// `flag` (or-ed in).  LOW's branch keeps the compiler from mixing what stands
-// before and after it: k_edge_final takes 0.5 % longer with it, k_aux2 3 % and
-// k_cell_tracers with 8 tracers 8 % (630 -> 681 us at 256x256x64).
-template <int N, bool LOW>
+// FX_FLAG is set, or with FX_LEAVE where fx_left says so, which is reported in
+// `flag` (or-ed in).  FX_RESOLVE is for any weights and values, and what the
+// others are tested beside; no pass takes it, as its branch keeps the compiler
+// from mixing what stands before and after it: k_aux2 takes 3 %
+// longer with it, k_cell_tracers with 8 tracers 8 % (630 -> 681 us at
+// 256x256x64) and the batched edge pass 6 %.  FX_LEAVE takes 0.8, 0 and 4 %.
+template <int N, FxZeros Z>
 SWG_HD double fx_sum(const Wt (&w)[N], const fx_t (&x)[N], long long start,
                      int top, unsigned &flag) {
   static_assert(N <= 14, "the 64-bit accumulators hold 14 products");
   int p[N];
   unsigned f;
   int P = fx_exps(w, x, p, f);
-  if (!LOW) {
-    flag |= fx_left(P, top, f);
-  } else {
-    if (P <= top && f != 0) {
-      P = FX_ZERO_EXP;
+  if (Z == FX_RESOLVE && P <= top && f != 0) {
+    P = FX_ZERO_EXP;
 #pragma unroll
-      for (int j = 0; j < N; ++j)
-        P = unsigned(x[j]) != 0 && p[j] > P ? p[j] : P;
-    }
-    flag |= f & FX_FLAG;
+    for (int j = 0; j < N; ++j)
+      P = unsigned(x[j]) != 0 && p[j] > P ? p[j] : P;
   }
+  // (each flag where the sums of its passes are the faster: 634 -> 630 us for
+  // k_cell_tracers, 318 -> 304 us for the edge pass of 12 members)
+  if (Z == FX_LEAVE)
+    flag |= fx_left(P, top, f);
   FxAcc a{0, 0, start};
 #pragma unroll
   for (int j = 0; j < N; ++j)
     fx_mac(a, w[j], x[j], P, p[j]);
+  if (Z != FX_LEAVE)
+    flag |= f & FX_FLAG;
   return fx_finish(a, P);
 }
 template <int N>
 SWG_HD double fx_sum(const Wt (&w)[N], const fx_t (&x)[N], long long start,
                      unsigned &flag) {
-  return fx_sum<N, true>(w, x, start, fx_top(w), flag);
+  return fx_sum<N, FX_RESOLVE>(w, x, start, fx_top(w), flag);
 }
 
 // ---- sums of float64 values as they are

@@ -225,11 +225,75 @@ extern "C" double sum12(const double *w, const double *x, unsigned *flag) {
     X[j] = fx_word(x[j]);
     s += W[j].hi;
   }
-  double r = fx_sum<12, false>(W, X, fx_start(s), FX_TOP, f);
+  double r = fx_sum<12, FX_LEAVE>(W, X, fx_start(s), FX_TOP, f);
   *flag = f;
   return r;
 }
 """
+
+
+PV_SRC = r"""
+#include "swg_fixed.cuh"
+using namespace swg;
+extern "C" unsigned long long word(double x) { return fx_word<FX_PV_MINQ>(x); }
+extern "C" int spread() { return FX_PV_SPREAD; }
+extern "C" double sum8(const double *w, const double *x, unsigned *flag) {
+  Wt W[8];
+  fx_t X[8];
+  long long s = 0;
+  unsigned f = 0;
+  for (int j = 0; j < 8; ++j) {
+    W[j] = fx_weight(w[j], f);
+    X[j] = fx_word<FX_PV_MINQ>(x[j]);
+    s += W[j].hi;
+  }
+  double r = fx_sum<8, FX_NONE>(W, X, fx_start(s), FX_TOP, f);
+  *flag = f;
+  return r;
+}
+"""
+
+
+def test_pv_sums_need_no_look_at_zeros(tmp_path):
+    """The PV sums' words: with weights within their spread of each other the
+    bound holds for every mixture of zeros and values down to the smallest
+    word; smaller values are flagged."""
+    src, so = tmp_path / "pv.cpp", tmp_path / "pv.so"
+    src.write_text(PV_SRC)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC,
+                    "-o", str(so), str(src)], check=True)
+    lib = ctypes.CDLL(str(so))
+    lib.sum8.restype = ctypes.c_double
+    lib.sum8.argtypes = [ctypes.POINTER(ctypes.c_double),
+                         ctypes.POINTER(ctypes.c_double),
+                         ctypes.POINTER(ctypes.c_uint)]
+    lib.word.restype = ctypes.c_uint64
+    lib.word.argtypes = [ctypes.c_double]
+    least = 2.0**-293
+    for x in (least, -least, 1.5 * least, 2.0**66, 0.0):
+        assert not lib.word(x) & 0x80
+    for x in (math.nextafter(least, 0.0), -least / 2, 2.0**-314, 5e-324, 2.0**67,
+              math.inf, math.nan):
+        assert lib.word(x) & 0x80
+    spread = lib.spread()
+    rng = random.Random(8)
+    for trial in range(6000):
+        w = [rng.choice((-1, 1)) * (1 + rng.random())
+             * 2.0**(rng.randint(0, spread) if rng.random() < 0.7
+                     else rng.choice((0, spread))) for _ in range(8)]
+        x = [rng.choice((-1, 1)) * (1 + rng.random())
+             * 2.0**-rng.randint(293 - trial % 2 * 9, 293) for _ in range(8)]
+        for _ in range(rng.randint(0, 7)):
+            x[rng.randrange(8)] = 0.0
+        if trial % 3 == 0:
+            w[rng.randrange(8)] = 0.0
+        r, flag = _sum(lib, w, x)
+        assert flag == 0
+        prods = [Fraction(a) * Fraction(b) for a, b in zip(w, x)]
+        exact, M = sum(prods), max(abs(p) for p in prods)
+        tol = (8 * (Fraction(1, 2**56) + Fraction(1, 2**59))
+               + Fraction(1, 2**56)) * M + Fraction(1, 2**53) * abs(exact)
+        assert abs(Fraction(r) - exact) <= tol * Fraction(1001, 1000)
 
 
 def test_sums_that_leave_small_products_to_fp64(tmp_path):
