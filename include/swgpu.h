@@ -356,9 +356,10 @@ int swg_host_free(void *p);
  * runs one instance per process; each member's step is the reference's
  * do_step).  Members are (model, state) pairs whose models have no forcing
  * hook and share the edges-on-edge width; the batch owns the stepper scratch
- * of every member.  One RK stage of all members is one persistent
- * cooperative kernel (six passes separated by bounded grid barriers), or one
- * launch per pass, whichever launch configuration is selected. */
+ * of every member.  One RK stage of all members is one launch per pass (a new
+ * batch's configuration), or one persistent cooperative kernel (passes
+ * separated by bounded grid barriers) with launches of their own for the passes
+ * whose sums are fixed-point, whichever launch configuration is selected. */
 /* The batch keeps the member handles (and a CUDA graph of their device
  * arrays): the models and states must outlive it, and no model or state may
  * appear in two members (SWG_ERR_ARG). */

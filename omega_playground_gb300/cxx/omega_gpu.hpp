@@ -692,7 +692,7 @@ struct HostStepper {
 // Beside the plain solver; no counterpart in the reference.
 
 // Many independent members (own mesh size, levels and tracers) advanced
-// together: one persistent kernel, or one launch per pass, per RK stage
+// together: one launch per pass, or one persistent kernel, per RK stage
 // (swg_batch_*).  Members must have distinct models and states, and those
 // must outlive the stepper (it keeps their handles).
 struct EnsembleStepper {

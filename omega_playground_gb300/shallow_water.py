@@ -803,7 +803,8 @@ class HostStepper:
 
 class Batch:
     """Ensemble of independent members (uneven nx, levels, tracers) advanced
-    together by one persistent kernel per RK stage (swg_batch_* in swgpu.h).
+    together by one launch per pass of an RK stage, or one persistent kernel
+    (swg_batch_* in swgpu.h).
     Members are (ShallowWaterModel, ShallowWaterState) pairs."""
 
     def __init__(self, models, states, kind: str = "rk4", nstages: int = 4):
