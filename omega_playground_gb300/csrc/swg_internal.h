@@ -336,10 +336,10 @@ namespace swg {
 // of them; below FX_MIN_LEVELS levels its lanes belong to many entities, and
 // the 16-byte entries of the PV sums cost more than the FP64 instructions
 // they save (edge pass, 65536 cells: 1 level 16.3 us in FP64, 18.7 fixed; 2
-// levels 17.7 and 16.2; 4 levels 22.4 and 18.7).  In batches whose larger
-// members have 2 to 4 levels the sums do not pay: members without words share
-// the word passes' launches (6 members to 170x170x3, no tracers: 794 us in FP64,
-// 851 fixed; single steps of 160x160x3 1.06 times as fast).  Size: the edge pass
+// levels 17.7 and 16.2; 4 levels 22.4 and 18.7).  In batches of uneven
+// members with 2 to 4 levels the sums do not pay (6 members to 170x170x3, no
+// tracers: 794 us in FP64, 815 fixed; of one size 1324 and 1286), but a batch
+// sums as single steps do, which gain (160x160x3: 1.06).  Size: the edge pass
 // keeps 28 warps per SM resident, 136k threads (24 and 117k in batches); a model
 // with fewer edge-levels does not fill them, and the longer chain of a sum shows
 // (RK4 step, 1 tracer, 48x48 cells x 16 levels: 77.5 us in FP64, 80.2 fixed;
