@@ -33,9 +33,9 @@
 // more than a bound `top` of the e_j and some word is not zero, the sum leaves
 // the zeros' exponents out, or it is left to FP64 with those below; or it
 // cannot happen, with weights that lie within FX_PV_SPREAD binades of each
-// other and words of values not so small (fx_word<FX_PV_MINQ>).  The passes
-// take weights below 2^36 and the constant FX_TOP: only sums with M below
-// 2^-278 are looked at again.
+// other and words of values not so small (fx_word<FX_PV_MINQ>).  The tracer
+// passes take weights below 2^36 and the constant FX_TOP: only sums with M
+// below 2^-278 are left to FP64.
 //
 // A term that cannot be represented (a flagged word, or a weight out of
 // range) makes the caller evaluate that one sum in FP64 instead: infinities
@@ -57,7 +57,7 @@ using fx_t = unsigned long long;
 constexpr unsigned FX_FLAG = 0x80; // low-byte bit of an unrepresentable value
 constexpr int FX_ZERO_EXP = -100000; // exponent of a zero weight
 constexpr int FX_BAD_EXP = 100000;   // and of a table's out-of-range weight
-constexpr int FX_TOP = -20;          // largest exponent of a pass's weight
+constexpr int FX_TOP = -20;          // largest exponent of a tracer weight
 constexpr int FX_PV_MINQ = 8;        // smallest q of a word of the PV sums, and
 constexpr int FX_PV_SPREAD = 3 * FX_PV_MINQ - 1; // what their weights differ by
 constexpr int FX_SCALE = -317;       // 60 - 377: result exponent offset
